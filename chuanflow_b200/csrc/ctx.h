@@ -199,6 +199,32 @@ private:
     int uPrecond_ = CFG_PRECOND_JACOBI;
     float* uVal32_ = nullptr;
     void launchCheck(const char* what, int kernels = 1);
+    /// The team of blocks a whole Krylov solve runs in as one kernel
+    /// (persist.cuh): no team (blocks 0: the per-iteration kernels), a
+    /// cluster or a cooperative grid, rows per thread and rows per block.
+    struct TeamPlan
+    {
+        int blocks = 0;  // per team
+        bool cluster = false;
+        int NC = 1;      // components per team
+        int K = 0, chunk = 0;
+    };
+    TeamPlan teamPlan(int nComp, bool bicg) const;
+    template <class Kern, class A>
+    void teamLaunch(const TeamPlan& tp, int teams, Kern kernel, const A& args, size_t smem, double tol, int maxIter, int normType);
+    void teamBi(const TeamPlan& tp, int nComp, const double* vals, const double* diag, V3P b, V3P x, double tol,
+                int maxIter);
+    template <bool kDic>
+    void teamCg(const TeamPlan& tp, const double* vals, const double* diag, const double* b, double* x,
+                const double* rDinv, double tol, int maxIter, int normType);
+    void teamReport(int nComp, cfg_solver_report* reps);
+    void checkTeam() const;
+    int clusterMax_ = 0;            // largest cluster this device runs
+    bool coopOk_ = false;           // cooperative launches
+    int* dColour_ = nullptr;        // DIC colour of each row
+    unsigned* teamCount_ = nullptr; // a grid team's counters
+    double* teamPart_ = nullptr;    // and partials
+    int* teamFailed_ = nullptr;     // host-mapped: a grid team's wait ran out
     int linUpwindGrad(const BcTab& ub, int gradScheme);
     template <class F>
     void launchChunk(const std::string& key, int n, F&& body);

@@ -1074,7 +1074,10 @@ void Ctx::mpnnFcg(const double* vals, const double* diag, const double* b, doubl
     {
         cfg_solver_report rep{};
         if (normType == 0) dicSetup(vals, diag);  // the SIMPLE/PISO matrix of this solve
+        double* const tally = tally_;  // its outcome is read here, not left to the outer iteration's tally
+        tally_ = nullptr;
         dicCGT<double>(dic_, vals, diag, b, x, cr_, cp_, cAp_, cz_, tol, maxIter - it, normType, &rep);
+        tally_ = tally;
         out[1] = rep.iterations;
         out[2] = 1;
     }

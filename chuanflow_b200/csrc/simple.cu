@@ -5,12 +5,15 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <type_traits>
 
 #include "ctx.h"
 #include "kernels.cuh"
 #include "solvers.cuh"
 #include "dic.cuh"
+#include "persist.cuh"
 
 namespace cfg
 {
@@ -624,12 +627,50 @@ Ctx::~Ctx()
     for (void* p : allocs_) cudaFree(p);
     if (stHost_) cudaFreeHost(stHost_);
     if (scalHost_) cudaFreeHost(scalHost_);
+    if (teamFailed_) cudaFreeHost(teamFailed_);
     for (int i = 0; i < 16; ++i) cudaEventDestroy(tm_.ev[i]);
     for (auto& e : kev_) cudaEventDestroy(e);
     for (auto& g : graphs_) cudaGraphExecDestroy(g.second);
     if (bodyStream_) cudaStreamDestroy(bodyStream_);
     if (ownStream_) cudaStreamDestroy(stream_);
 }
+
+namespace
+{
+/// The largest cluster of whole-solve blocks the device runs: 16 (a
+/// non-portable size, which a partitioned GPU may not have), else 8, else 0.
+int largestCluster(int device)
+{
+    static std::mutex mu;
+    static std::map<int, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    const auto it = known.find(device);
+    if (it != known.end()) return it->second;
+    const auto kernel = k_pers_cg<4, ClusterTeam, true>;
+    const size_t smem = resident_smem(4, 1, false);
+    int best = 0;
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+        cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess)
+        for (int size = kClusterMax; size >= 8 && best == 0; size /= 2)
+        {
+            cudaLaunchConfig_t cfg{};
+            cfg.gridDim = dim3(static_cast<unsigned>(size));
+            cfg.blockDim = dim3(kTeamThreads);
+            cfg.dynamicSmemBytes = smem;
+            cudaLaunchAttribute at[1];
+            at[0].id = cudaLaunchAttributeClusterDimension;
+            at[0].val.clusterDim.x = static_cast<unsigned>(size);
+            at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+            cfg.attrs = at;
+            cfg.numAttrs = 1;
+            int clusters = 0;
+            if (cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0) best = size;
+        }
+    cudaGetLastError();  // a refused size is an answer, not an error
+    known[device] = best;
+    return best;
+}
+}  // namespace
 
 void Ctx::buildDevice()
 {
@@ -866,6 +907,13 @@ void Ctx::buildDevice()
         }
         dicPartials_ = pOff + 1;
         initDicPartials_ = dicPartials_;
+        {
+            std::vector<int> colour(static_cast<size_t>(nC), 0);
+            for (size_t c = 0; c < dicPhase_.size(); ++c)
+                for (int t = 0; t < dicPhase_[c].cnt; ++t)
+                    colour[static_cast<size_t>(rows[static_cast<size_t>(dicPhase_[c].off + t)])] = static_cast<int>(c);
+            dColour_ = upload(colour);
+        }
         dic_.nColours = nCol;
         dic_.rows = upload(rows);
         dic_.lStart = upload(lStart);
@@ -996,6 +1044,16 @@ void Ctx::buildDevice()
     CFG_CUDA(cudaStreamCreateWithFlags(&bodyStream_, cudaStreamNonBlocking));
     CFG_CUDA(cudaMallocHost(&stHost_, sizeof(SolveState)));
     CFG_CUDA(cudaMallocHost(&scalHost_, sizeof(double) * S_COUNT));
+    teamCount_ = alloc<unsigned>(kTeamsMax * kCountStride);
+    teamPart_ = alloc<double>(kTeamsMax * 2 * kTeamVals * (static_cast<size_t>(nC) / kGroupRows + 1));
+    clusterMax_ = largestCluster(device_);
+    {
+        int coop = 0;
+        CFG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device_));
+        coopOk_ = coop != 0;
+    }
+    CFG_CUDA(cudaHostAlloc(&teamFailed_, sizeof(int), cudaHostAllocMapped));
+    *teamFailed_ = 0;
     CFG_CUDA(cudaStreamSynchronize(stream_));
 }
 
@@ -1407,10 +1465,169 @@ std::string ptrKey(const char* kind, std::initializer_list<const void*> ps, int 
 }
 }  // namespace
 
+namespace
+{
+// rows per thread that registers and shared memory hold: one component, and
+// the three-component BiCGStab
+constexpr int kRes1K = 4, kRes3K = 2;
+}  // namespace
+
+/// The team of a solve of nComp components, measured on jittered channels
+/// (Jacobi momentum and pressure, one outer iteration, B200; per-iteration
+/// kernels -> team): a cluster per component up to 16 blocks x 4 rows per
+/// thread = 32,768 rows (1,320 rows 31 -> 6.9 ms, 16,000 rows 138 -> 35 ms,
+/// 22,743 rows 45 -> 14 ms; a grid there took 20, 71 and 21 ms, its barriers
+/// costing six of a cluster's); then a grid per component while the rows fit
+/// (62,720 rows 73 -> 36 ms, 102,400 rows 93 -> 45 ms for the pair of
+/// solvers), then one grid for the three together (131,544 rows, DIC: 58 ->
+/// 33 ms).  Larger systems stream from memory anyway and keep the
+/// per-iteration kernels.  Detail blocks and captured passes run side by
+/// side with others on the device and never take a grid, which wants every
+/// SM at once: their clusters do not depend on the schedule.
+Ctx::TeamPlan Ctx::teamPlan(int nComp, bool bicg) const
+{
+    TeamPlan tp;
+    // per-kernel event timing needs the per-iteration kernels; longer rows
+    // do not fit the resident layout
+    if (ktime_ || maxW_ > kResW) return tp;
+    const int n = dm_.nC;
+    // rows per block in whole groups of 256 (the unit of a sum's order)
+    const int groups = (n + kGroupRows - 1) / kGroupRows;
+    auto perBlock = [&](int blocks) { return (groups + blocks - 1) / blocks; };
+    // more groups than team_final_sum adds; a scalar equation's sums keep the
+    // per-iteration kernels' order, which has one row per thread up to G rows
+    if (groups > 768 || (bicg && nComp == 1 && n > initGS_ * TPB)) return tp;
+    auto perThread = [&](int blocks) { return (perBlock(blocks) * kGroupRows + kTeamThreads - 1) / kTeamThreads; };
+    const bool gridOk = coopOk_ && !detail_ && !devLoop_;
+    if (clusterMax_ > 0 && perThread(clusterMax_) <= kRes1K)
+    {
+        tp.cluster = true;
+        tp.blocks = 1;
+        while (tp.blocks < clusterMax_ && perThread(tp.blocks) > 1) tp.blocks *= 2;
+    }
+    else if (gridOk && perThread(sms_ / nComp) <= kRes1K)
+        tp.blocks = sms_ / nComp;
+    else if (gridOk && nComp == 3 && perThread(sms_) <= kRes3K)
+    {
+        tp.blocks = sms_;
+        tp.NC = 3;
+    }
+    if (tp.blocks)
+    {
+        tp.K = perThread(tp.blocks);
+        tp.chunk = perBlock(tp.blocks) * kGroupRows;
+    }
+    return tp;
+}
+
+/// Launches a whole-solve kernel as its team.
+template <class Kern, class A>
+void Ctx::teamLaunch(const TeamPlan& tp, int teams, Kern kernel, const A& args, size_t smem, double tol, int maxIter,
+                     int normType)
+{
+    const PersArgs t{tol, maxIter, normType, tp.chunk, st_, tally_, {tp.blocks, teamCount_, teamPart_,
+                     (dm_.nC + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, teamFailed_}};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(tp.blocks * teams));
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream_;
+    cudaLaunchAttribute at[1];
+    CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (tp.cluster)
+    {
+        if (tp.blocks > 8) CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = static_cast<unsigned>(tp.blocks);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    }
+    else
+    {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CFG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args, t));
+    launchCheck("team_solve");
+}
+
+namespace
+{
+/// f(std::integral_constant<int, K>) for 1 <= K <= Kmax
+template <int Kmax, class F>
+void dispatchK(int K, F&& f)
+{
+    if constexpr (Kmax > 1)
+        if (K < Kmax) return dispatchK<Kmax - 1>(K, f);
+    f(std::integral_constant<int, Kmax>{});
+}
+}  // namespace
+
+void Ctx::teamBi(const TeamPlan& tp, int nComp, const double* vals, const double* diag, V3P b, V3P x, double tol,
+                 int maxIter)
+{
+    const PersBi a{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag, b, x, bz_};
+    if (tp.NC == 3)
+        dispatchK<kRes3K>(tp.K, [&](auto Kc) {
+            constexpr int K = decltype(Kc)::value;
+            teamLaunch(tp, 1, k_pers_bicg<K, GridTeam, 3>, a, resident_smem(K, 3, false), tol, maxIter, 0);
+        });
+    else
+        dispatchK<kRes1K>(tp.K, [&](auto Kc) {
+            constexpr int K = decltype(Kc)::value;
+            const size_t smem = resident_smem(K, 1, false);
+            if (tp.cluster) teamLaunch(tp, nComp, k_pers_bicg<K, ClusterTeam, 1>, a, smem, tol, maxIter, 0);
+            else teamLaunch(tp, nComp, k_pers_bicg<K, GridTeam, 1>, a, smem, tol, maxIter, 0);
+        });
+}
+
+template <bool kDic>
+void Ctx::teamCg(const TeamPlan& tp, const double* vals, const double* diag, const double* b, double* x,
+                 const double* rDinv, double tol, int maxIter, int normType)
+{
+    const PersCg a{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag, b, x, cp_, rDinv, dColour_, dic_.nColours};
+    dispatchK<kRes1K>(tp.K, [&](auto Kc) {
+        constexpr int K = decltype(Kc)::value;
+        if (tp.cluster) teamLaunch(tp, 1, k_pers_cg<K, ClusterTeam, kDic>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
+        else teamLaunch(tp, 1, k_pers_cg<K, GridTeam, kDic>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
+    });
+}
+
+/// The outcome of a whole-solve kernel: left to the device's tally inside an
+/// outer iteration (nothing waits), else read here.
+void Ctx::teamReport(int nComp, cfg_solver_report* reps)
+{
+    for (int q = 0; q < nComp; ++q) reps[q] = cfg_solver_report{};
+    if (tally_ || devLoop_) return;
+    CFG_CUDA(cudaMemcpyAsync(stHost_, st_, sizeof(SolveState), cudaMemcpyDeviceToHost, stream_));
+    CFG_CUDA(cudaStreamSynchronize(stream_));
+    checkTeam();
+    for (int q = 0; q < nComp; ++q)
+    {
+        reps[q].iterations = stHost_->it[q];
+        reps[q].converged = stHost_->conv[q];
+        reps[q].initial_residual = stHost_->init[q];
+        reps[q].final_residual = stHost_->fin[q];
+    }
+}
+
+void Ctx::checkTeam() const
+{
+    if (*static_cast<volatile int*>(teamFailed_))
+        fail(CFG_ECUDA, "solver: a grid barrier's wait ran out");
+}
+
 void Ctx::runCG(const double* vals, const double* diag, const double* b, double* x, double tol, int maxIter,
                 cfg_solver_report* rep, int normType)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
+    if (const TeamPlan tp = teamPlan(1, false); tp.blocks)
+    {
+        teamCg<false>(tp, vals, diag, b, x, nullptr, tol, maxIter, normType);
+        teamReport(1, rep);
+        return;
+    }
     SolveState init{};
     init.tol = tol;
     init.maxIter = maxIter;
@@ -1485,6 +1702,12 @@ void Ctx::runBiCG3(const double* vals, const double* diag, V3P b, V3P x, int nCo
                    cfg_solver_report* reps)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
+    if (const TeamPlan tp = teamPlan(nComp, true); tp.blocks)
+    {
+        teamBi(tp, nComp, vals, diag, b, x, tol, maxIter);
+        teamReport(nComp, reps);
+        return;
+    }
     SolveState init{};
     init.tol = tol;
     init.maxIter = maxIter;
@@ -1713,6 +1936,15 @@ void Ctx::dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T*
                  double tol, int maxIter, int normType, cfg_solver_report* rep)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
+    if constexpr (std::is_same<T, double>::value)
+    {
+        if (const TeamPlan tp = teamPlan(1, false); tp.blocks)
+        {
+            teamCg<true>(tp, vals, diag, b, x, D.rDinv, tol, maxIter, normType);
+            teamReport(1, rep);
+            return;
+        }
+    }
     SolveState init{};
     init.tol = tol;
     init.maxIter = maxIter;
@@ -2313,6 +2545,7 @@ void Ctx::enqueueOuter(const cfg_simple_controls& ctl, int64_t& uInner, int64_t&
 int Ctx::finishOuter(const cfg_simple_controls& ctl, int iter, double& contLag1, double& contLag2,
                      cfg_simple_result& res)
 {
+    checkTeam();
     const double* S = scalHost_;
     const double contErr = S[S_CONT], errAfter = S[S_CONT_AFTER], pDeltaMax = S[S_PDELTA];
     const double uRes = S[S_DUMAX] / std::max(S[S_UMAX], 1e-300);
@@ -2363,6 +2596,12 @@ void Ctx::iterate(const cfg_simple_controls& ctl, cfg_simple_result& res)
     {
         enqueueOuter(ctl, res.u_inner_iterations, res.p_inner_iterations);
         CFG_CUDA(cudaStreamSynchronize(stream_));
+        // what the whole-solve kernels counted on the device
+        int64_t u = 0, p = 0, t = 0;
+        deviceInner(u, p, t);
+        res.u_inner_iterations += u;
+        res.p_inner_iterations += p;
+        lastTurbInner += t;
         if (finishOuter(ctl, iter, contLag1, contLag2, res)) break;
     }
     CFG_CUDA(cudaEventRecord(tm_.ev[1], stream_));
@@ -2376,6 +2615,7 @@ void Ctx::iterate(const cfg_simple_controls& ctl, cfg_simple_result& res)
 /// solveTransientIncompressiblePiso (pisoSolver.cpp:13-237), one time step
 void Ctx::pisoStep(const cfg_piso_controls& ctl, cfg_piso_result& res)
 {
+    tally_ = nullptr;
     CFG_CUDA(cudaSetDevice(device_));
     if (!(ctl.dt > 0)) fail(CFG_EINVAL, "PISO: non-positive time step");
     refreshBc();
@@ -2778,6 +3018,7 @@ void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3])
 void Ctx::poissonSolve(const double* b, double* x, int method, double tol, int maxIter, int innerMax, double innerTol,
                        double* out)
 {
+    tally_ = nullptr;
     // out: inner iterations, outer iterations, converged, true |b-Ax|2/|b|2,
     //      device ms, initial true relative residual
     if (!poissonReady_) fail(CFG_EINVAL, "cfg_poisson_solve: call cfg_poisson_setup first");
