@@ -17,12 +17,13 @@
 // densely on the host (diagonally regularised when singular, as a pure
 // Neumann system is).
 //
-// V-cycle (device, FP32 vectors and values): per level one kernel does the
-// first damped-Jacobi sweep from zero and the residual, one sums the
-// residual over each aggregate, and after the coarse solve one kernel adds
-// the coarse correction (scaled by s > 1, which makes up for the piecewise
-// constant interpolation) and does the last Jacobi sweep.  The finest level
-// reads the FCG residual in FP64 and writes z in FP64.
+// V-cycle (device, FP32 vectors and values): on the finest level one kernel
+// does a damped-Jacobi sweep from zero and the residual; the residual is
+// summed over each aggregate; the coarse levels sweep, correct and sweep
+// again, one to four weighted sweeps each time (smootherOf); a correction is
+// scaled by s > 1, which makes up for the piecewise constant interpolation;
+// and one kernel does the finest level's last sweep.  The finest level reads
+// the FCG residual in FP64 and writes z in FP64.
 #include <algorithm>
 #include <chrono>
 #include <cmath>
@@ -37,6 +38,23 @@
 
 namespace cfg
 {
+
+/// m Jacobi sweeps and their weights: w[0], w[1], ... before a coarse
+/// correction, in reverse after it.
+constexpr int kSweepsMax = 4;
+struct Sweeps
+{
+    int m = 1;
+    float w[kSweepsMax] = {};
+};
+
+/// The sweeps of the first coarse level and of the levels below it (the
+/// finest has one of weight kOmega on either side).
+struct Smoother
+{
+    Sweeps first, rest;
+    const Sweeps& at(int level) const { return level <= 1 ? first : rest; }
+};
 
 struct AmgLevel
 {
@@ -61,8 +79,8 @@ struct AmgLevel
     float* sval = nullptr;
     // work vectors: rhs, first sweep, residual, output
     float *b = nullptr, *x = nullptr, *r = nullptr, *xo = nullptr;
-    // the same for the three-component V-cycle (a float4 per row above the
-    // last level, component q at q * n on it), allocated on its first use
+    // the same for the three-component V-cycle (a float4 per row), allocated
+    // on its first use
     float *b3 = nullptr, *x3 = nullptr, *r3 = nullptr, *xo3 = nullptr;
 };
 
@@ -94,10 +112,12 @@ struct AmgState
     double setupMs = 0, valuesMs = 0;
     double theta = 0;                 // strength threshold of the aggregation (0: plain)
     const float* vals32 = nullptr;    // the finest operator's FP32 SELL values
-    // the tail level in shared memory: the dynamic size (0: it does not
-    // fit, k_amg_tail runs from global memory) and the level's entries
+    // k_amg_tail: the dynamic shared memory of the last aggregated level and
+    // its entries (0: it does not fit, its kernels and k_amg_dense run)
     size_t tailSmem = 0;
     int tailNnz = 0;
+    int skewClass = 0;    // how far from symmetric the finest operator is (skewOf)
+    double* skew = nullptr;
 };
 
 void AmgDeleter::operator()(AmgState* a) const { delete a; }
@@ -111,6 +131,30 @@ constexpr int kDenseMax = 128;
 // coarse levels of at least this many rows keep a SELL-32 copy of their
 // operator: one thread per row fills the GPU in one wave there
 constexpr int kSellMinRows = 32768;
+
+/// m sweeps whose product is the Chebyshev polynomial of [lo, hi] in D^-1 A
+Sweeps chebyshev(int m, double lo, double hi)
+{
+    Sweeps s;
+    s.m = m;
+    for (int k = 0; k < m; ++k)
+        s.w[k] = static_cast<float>(1.0 / (0.5 * (hi + lo) + 0.5 * (hi - lo) * std::cos(M_PI * (2 * k + 1) / (2.0 * m))));
+    return s;
+}
+Sweeps jacobi(int m)
+{
+    Sweeps s;
+    s.m = m;
+    for (int k = 0; k < m; ++k) s.w[k] = kOmega;
+    return s;
+}
+/// one sweep before and after each correction on every level
+Smoother singleSweeps() { return Smoother{jacobi(1), jacobi(1)}; }
+
+/// The class of a nonsymmetric operator by theta = max over rows of
+/// sum_j |a_ij - a_ji| / (2 a_ii), a bound of the imaginary parts of D^-1 A:
+/// Chebyshev sweeps amplify eigenvalues far off the real axis.
+int skewOf(double theta) { return theta <= 0.5 ? 0 : (theta <= 0.9 ? 1 : 2); }
 
 /// One full wave of a grid-stride row kernel of TPB threads: the SMs times
 /// the blocks of this kernel one SM holds at once (its registers decide),
@@ -188,37 +232,6 @@ __device__ __forceinline__ float sell_row(const DMat& A, const float* __restrict
     return s;
 }
 
-/// a CSR row of a coarse level summed by a group of G lanes (rows there are
-/// long and few): lane l of the group takes entries l, l + G, ...; the
-/// group's lanes hold the sum after the shuffle tree
-template <int G, class F>
-__device__ __forceinline__ float group_row(const int* __restrict__ rs, const int* __restrict__ cols,
-                                           const float* __restrict__ val, int i, int l, F f)
-{
-    float s = 0.0f;
-    if (i >= 0)
-        for (int e = __ldg(rs + i) + l; e < __ldg(rs + i + 1); e += G) s += __ldg(val + e) * f(__ldg(cols + e));
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
-}
-constexpr int kGroup = 4;
-
-/// the sum of an aggregate's members, by a group of G lanes: lane l of the
-/// group takes members l, l + G, ...; every lane of the group holds the
-/// sum after the shuffle tree
-template <int G>
-__device__ __forceinline__ float group_members(const int* __restrict__ ms, const int* __restrict__ mem,
-                                               const float* __restrict__ r, int I, int l)
-{
-    float s = 0.0f;
-    if (I >= 0)
-        for (int k = __ldg(ms + I) + l; k < __ldg(ms + I + 1); k += G) s += __ldg(r + __ldg(mem + k));
-#pragma unroll
-    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    return s;
-}
-
 /// finest level, first sweep and residual: x = w D^-1 b, r = b - A x
 template <int W>
 __global__ void __launch_bounds__(TPB) k_amg_pre0(const int* __restrict__ stop, DMat A, const float* __restrict__ val,
@@ -235,79 +248,6 @@ __global__ void __launch_bounds__(TPB) k_amg_pre0(const int* __restrict__ stop, 
             sell_row<W>(A, val, c, [&](int j) { return kOmega * __ldg(dinv + j) * static_cast<float>(__ldg(b + j)); });
         r[c] = bc - s;
     }
-}
-
-/// coarse level, the same on CSR, a group of G lanes per row
-template <int G>
-__device__ __forceinline__ void amg_pre_rows(int n, const int* __restrict__ rs, const int* __restrict__ cols,
-                                             const float* __restrict__ val, const float* __restrict__ dinv,
-                                             const float* __restrict__ b, float* __restrict__ x,
-                                             float* __restrict__ r, int first, int stride)
-{
-    const int l = threadIdx.x % G;
-    // whole warps iterate together (the shuffle needs every lane)
-    for (int i0 = first;; i0 += stride)
-    {
-        const int base = i0 - (threadIdx.x % 32) / G;  // the warp's first row this round
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        const float s = group_row<G>(rs, cols, val, i, l, [&](int j) { return kOmega * __ldg(dinv + j) * __ldg(b + j); });
-        if (i >= 0 && l == 0)
-        {
-            const float bi = b[i];
-            x[i] = kOmega * dinv[i] * bi;
-            r[i] = bi - s;
-        }
-    }
-}
-
-template <int G>
-__global__ void __launch_bounds__(TPB) k_amg_pre(const int* __restrict__ stop, int n, const int* __restrict__ rs,
-                                                 const int* __restrict__ cols, const float* __restrict__ val,
-                                                 const float* __restrict__ dinv, const float* __restrict__ b,
-                                                 float* __restrict__ x, float* __restrict__ r)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    amg_pre_rows<G>(n, rs, cols, val, dinv, b, x, r, blockIdx.x * (TPB / G) + threadIdx.x / G, gridDim.x * (TPB / G));
-}
-
-/// the residual summed over each aggregate (a group of G lanes per
-/// aggregate): the next level's right-hand side
-template <int G>
-__device__ __forceinline__ void amg_restrict_rows(int nc, const int* __restrict__ ms, const int* __restrict__ mem,
-                                                  const float* __restrict__ r, float* __restrict__ bc, int first,
-                                                  int stride)
-{
-    const int l = threadIdx.x % G;
-    for (int I0 = first;; I0 += stride)
-    {
-        const int base = I0 - (threadIdx.x % 32) / G;
-        if (base >= nc) break;
-        const int I = I0 < nc ? I0 : -1;
-        const float s = group_members<G>(ms, mem, r, I, l);
-        if (I >= 0 && l == 0) bc[I] = s;
-    }
-}
-
-template <int G>
-__global__ void __launch_bounds__(TPB) k_amg_restrict(const int* __restrict__ stop, int nc, const int* __restrict__ ms,
-                                                      const int* __restrict__ mem, const float* __restrict__ r,
-                                                      float* __restrict__ bc)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    amg_restrict_rows<G>(nc, ms, mem, r, bc, blockIdx.x * (TPB / G) + threadIdx.x / G, gridDim.x * (TPB / G));
-}
-
-/// the coarse correction brought to this level: y = x + s P xc
-__global__ void __launch_bounds__(TPB) k_amg_prolong(const int* __restrict__ stop, int n, const float* __restrict__ x,
-                                                     const float* __restrict__ xc, const int* __restrict__ agg,
-                                                     float* __restrict__ y)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    FOR_ROWS(i, n) y[i] = x[i] + kScale * xc[agg[i]];
 }
 
 /// finest level: z = y + w D^-1 (b - A y), in FP64 out; inside the device
@@ -343,225 +283,6 @@ __global__ void __launch_bounds__(TPB) k_amg_post0(const int* __restrict__ stop,
     }
 }
 
-/// coarse level, the same on CSR: xo = y + w D^-1 (b - A y), a group of G
-/// lanes per row
-template <int G>
-__device__ __forceinline__ void amg_post_rows(int n, const int* __restrict__ rs, const int* __restrict__ cols,
-                                              const float* __restrict__ val, const float* __restrict__ dinv,
-                                              const float* __restrict__ b, const float* __restrict__ y,
-                                              float* __restrict__ xo, int first, int stride)
-{
-    const int l = threadIdx.x % G;
-    for (int i0 = first;; i0 += stride)
-    {
-        const int base = i0 - (threadIdx.x % 32) / G;
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        const float s = group_row<G>(rs, cols, val, i, l, [&](int j) { return __ldg(y + j); });
-        if (i >= 0 && l == 0) xo[i] = y[i] + kOmega * dinv[i] * (b[i] - s);
-    }
-}
-
-template <int G>
-__global__ void __launch_bounds__(TPB) k_amg_post(const int* __restrict__ stop, int n, const int* __restrict__ rs,
-                                                  const int* __restrict__ cols, const float* __restrict__ val,
-                                                  const float* __restrict__ dinv, const float* __restrict__ b,
-                                                  const float* __restrict__ y, float* __restrict__ xo)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    amg_post_rows<G>(n, rs, cols, val, dinv, b, y, xo, blockIdx.x * (TPB / G) + threadIdx.x / G, gridDim.x * (TPB / G));
-}
-
-/// The last aggregation level (at most kTailMax rows) and the coarsest
-/// solve in one block per vector: pre-sweep and residual, restriction,
-/// the dense coarsest inverse, prolongation and post-sweep, separated by
-/// block barriers only (the same arithmetic and orders as the per-level
-/// kernels).  Block q works on vector q (offset q * n at every level) and
-/// does nothing when done[q] is set (done may be null).
-constexpr int kTailMax = 1024;
-constexpr int kTailThreads = 1024;
-
-struct TailLevel
-{
-    int n, nc;
-    const int *rs, *cols, *agg, *ms, *mem;
-    const float *val, *dinv, *dense;
-    float *b, *x, *r, *y, *xo;  // this level's vectors (n per vector)
-    float *bc, *xc;             // the coarsest level's (nc per vector)
-    float scale;                // coarse-correction scaling
-};
-
-__global__ void __launch_bounds__(kTailThreads) k_amg_tail(const int* __restrict__ done, TailLevel T)
-{
-    pdl_entry();
-    const int q = blockIdx.x;
-    if (done && done[q]) return;
-    const int n = T.n, nc = T.nc;
-    float *b = T.b + q * n, *x = T.x + q * n, *r = T.r + q * n, *y = T.y + q * n, *xo = T.xo + q * n;
-    float *bc = T.bc + q * nc, *xc = T.xc + q * nc;
-    const int first = threadIdx.x / kGroup, stride = kTailThreads / kGroup;
-    amg_pre_rows<kGroup>(n, T.rs, T.cols, T.val, T.dinv, b, x, r, first, stride);
-    __syncthreads();
-    amg_restrict_rows<kGroup>(nc, T.ms, T.mem, r, bc, first, stride);
-    __syncthreads();
-    // the coarsest solve xc = M bc: a warp per row, its lanes over the
-    // columns (coalesced reads of the inverse), then a shuffle tree
-    {
-        const int lane = threadIdx.x & 31;
-        for (int i = threadIdx.x >> 5; i < nc; i += kTailThreads / 32)
-        {
-            float s = 0.0f;
-            for (int j = lane; j < nc; j += 32) s += T.dense[i * nc + j] * bc[j];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) xc[i] = s;
-        }
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < n; i += kTailThreads) y[i] = x[i] + T.scale * xc[T.agg[i]];
-    __syncthreads();
-    amg_post_rows<kGroup>(n, T.rs, T.cols, T.val, T.dinv, b, y, xo, first, stride);
-}
-
-/// Shared-memory layout of k_amg_tail_smem (4-byte words): the level's CSR
-/// (rs n + 1, cols nnz, val nnz), dinv n, agg n, the aggregates' member
-/// lists (ms nc + 1, mem n), the dense inverse nc * nc, and the vectors b,
-/// x, r (then y) n each, bc and xc nc each.
-__host__ __device__ constexpr size_t tailSmemWords(int n, int nnz, int nc)
-{
-    return static_cast<size_t>(n + 1) + 2 * static_cast<size_t>(nnz) + 2 * static_cast<size_t>(n) +
-           static_cast<size_t>(nc + 1) + static_cast<size_t>(n) + static_cast<size_t>(nc) * nc + 3 * static_cast<size_t>(n) +
-           2 * static_cast<size_t>(nc);
-}
-
-/// k_amg_tail with the level held in shared memory: one coalesced load of
-/// the level's matrix, aggregates, dense inverse and right-hand side, then
-/// every phase (pre-sweep and residual, restriction, dense solve,
-/// prolongation, post-sweep) reads shared memory only, with the same lane
-/// groups, orders and arithmetic as k_amg_tail.  Block q works on vector q;
-/// only the output xo goes back to global memory.
-__global__ void __launch_bounds__(kTailThreads) k_amg_tail_smem(const int* __restrict__ done, TailLevel T, int nnz)
-{
-    pdl_entry();
-    const int q = blockIdx.x;
-    if (done && done[q]) return;
-    extern __shared__ __align__(16) int tsm[];
-    const int n = T.n, nc = T.nc, t = threadIdx.x;
-    int* rs = tsm;
-    int* cols = rs + (n + 1);
-    float* val = reinterpret_cast<float*>(cols + nnz);
-    float* dinv = val + nnz;
-    int* agg = reinterpret_cast<int*>(dinv + n);
-    int* ms = agg + n;
-    int* mem = ms + (nc + 1);
-    float* dense = reinterpret_cast<float*>(mem + n);
-    float* b = dense + static_cast<size_t>(nc) * nc;
-    float* x = b + n;
-    float* r = x + n;
-    float* bc = r + n;
-    float* xc = bc + nc;
-    for (int i = t; i <= n; i += kTailThreads) rs[i] = T.rs[i];
-    for (int e = t; e < nnz; e += kTailThreads)
-    {
-        cols[e] = T.cols[e];
-        val[e] = T.val[e];
-    }
-    for (int i = t; i < n; i += kTailThreads)
-    {
-        dinv[i] = T.dinv[i];
-        agg[i] = T.agg[i];
-        mem[i] = T.mem[i];
-        b[i] = T.b[static_cast<size_t>(q) * n + i];
-    }
-    for (int i = t; i <= nc; i += kTailThreads) ms[i] = T.ms[i];
-    for (int i = t; i < nc * nc; i += kTailThreads) dense[i] = T.dense[i];
-    __syncthreads();
-    const int l = t % kGroup, first = t / kGroup, stride = kTailThreads / kGroup;
-    // pre-sweep and residual: x = w D^-1 b, r = b - A x
-    for (int i0 = first;; i0 += stride)
-    {
-        const int base = i0 - (t % 32) / kGroup;
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        float s = 0.0f;
-        if (i >= 0)
-            for (int e = rs[i] + l; e < rs[i + 1]; e += kGroup)
-            {
-                const int j = cols[e];
-                s += val[e] * (kOmega * dinv[j] * b[j]);
-            }
-#pragma unroll
-        for (int o = kGroup / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (i >= 0 && l == 0)
-        {
-            x[i] = kOmega * dinv[i] * b[i];
-            r[i] = b[i] - s;
-        }
-    }
-    __syncthreads();
-    // restriction
-    for (int I0 = first;; I0 += stride)
-    {
-        const int base = I0 - (t % 32) / kGroup;
-        if (base >= nc) break;
-        const int I = I0 < nc ? I0 : -1;
-        float s = 0.0f;
-        if (I >= 0)
-            for (int k = ms[I] + l; k < ms[I + 1]; k += kGroup) s += r[mem[k]];
-#pragma unroll
-        for (int o = kGroup / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (I >= 0 && l == 0) bc[I] = s;
-    }
-    __syncthreads();
-    // the coarsest solve xc = M bc, a warp per row
-    {
-        const int lane = t & 31;
-        for (int i = t >> 5; i < nc; i += kTailThreads / 32)
-        {
-            float s = 0.0f;
-            for (int j = lane; j < nc; j += 32) s += dense[i * nc + j] * bc[j];
-#pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) xc[i] = s;
-        }
-    }
-    __syncthreads();
-    // prolongation into r (the residual is no longer needed)
-    for (int i = t; i < n; i += kTailThreads) r[i] = x[i] + T.scale * xc[agg[i]];
-    __syncthreads();
-    // post-sweep: xo = y + w D^-1 (b - A y)
-    float* xo = T.xo + static_cast<size_t>(q) * n;
-    for (int i0 = first;; i0 += stride)
-    {
-        const int base = i0 - (t % 32) / kGroup;
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        float s = 0.0f;
-        if (i >= 0)
-            for (int e = rs[i] + l; e < rs[i + 1]; e += kGroup) s += val[e] * r[cols[e]];
-#pragma unroll
-        for (int o = kGroup / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (i >= 0 && l == 0) xo[i] = r[i] + kOmega * dinv[i] * (b[i] - s);
-    }
-}
-
-/// the coarsest solve, x = M^-1 b with the dense inverse, when the finest
-/// level is the last aggregated one (block q: vector q at offset q * n)
-__global__ void __launch_bounds__(kDenseMax) k_amg_dense(const int* __restrict__ done, int n,
-                                                         const float* __restrict__ m, const float* __restrict__ b,
-                                                         float* __restrict__ x)
-{
-    pdl_entry();
-    const int q = blockIdx.x;
-    if (done && done[q]) return;
-    const int i = threadIdx.x;
-    if (i >= n) return;
-    float s = 0.0f;
-    for (int j = 0; j < n; ++j) s += m[i * n + j] * b[q * n + j];
-    x[q * n + i] = s;
-}
-
 /// next-level entries as sums of this level's: FP64 sums of FP64 (finest,
 /// SELL) or FP32 values, stored in FP32
 __global__ void __launch_bounds__(TPB) k_amg_galerkin(int nnz, const int* __restrict__ gs, const int* __restrict__ gl,
@@ -574,6 +295,47 @@ __global__ void __launch_bounds__(TPB) k_amg_galerkin(int nnz, const int* __rest
         for (int k = gs[e]; k < gs[e + 1]; ++k) s += fineD ? fineD[gl[k]] : static_cast<double>(fineF[gl[k]]);
         out[e] = static_cast<float>(s);
     }
+}
+
+/// max over rows of sum_j |a_ij - a_ji| / (2 a_ii), into the bits of *out
+__global__ void __launch_bounds__(TPB) k_amg_skew(DMat A, const double* __restrict__ val, unsigned long long* out)
+{
+    double mx[1] = {0.0};
+    FOR_ROWS(i, A.n)
+    {
+        const int e1 = __ldg(A.start + (i >> 5) + 1);
+        double s = 0.0, d = 0.0;
+        for (int e = __ldg(A.start + (i >> 5)) + (i & 31); e < e1; e += 32)
+        {
+            const int j = __ldg(A.col + e);
+            if (j < 0) break;
+            const double v = __ldg(val + e);
+            if (j == i)
+            {
+                d = v;
+                continue;
+            }
+            double w = 0.0;
+            const int f1 = __ldg(A.start + (j >> 5) + 1);
+            for (int f = __ldg(A.start + (j >> 5)) + (j & 31); f < f1; f += 32)
+            {
+                const int c = __ldg(A.col + f);
+                if (c < 0) break;
+                if (c == i)
+                {
+                    w = __ldg(val + f);
+                    break;
+                }
+            }
+            s += fabs(v - w);
+        }
+        const double t = d > 0.0 ? s / (2.0 * d) : 1.0;
+        if (!(t <= mx[0])) mx[0] = t;  // a NaN stays
+    }
+    // NaN counts as the worst
+    if (isnan(mx[0])) mx[0] = 1e300;
+    block_max<1>(mx);
+    if (threadIdx.x == 0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(mx[0])));
 }
 
 __global__ void __launch_bounds__(TPB) k_amg_dinv(int n, const int* __restrict__ dpos, const float* __restrict__ val,
@@ -648,27 +410,6 @@ __device__ __forceinline__ void sell_row3(const DMat& A, const float* __restrict
     }
 }
 
-/// a coarse CSR row against three vectors, summed by a group of G lanes
-template <int G, class F>
-__device__ __forceinline__ void group_row3(const int* __restrict__ rs, const int* __restrict__ cols,
-                                           const float* __restrict__ val, int i, int l, float (&s)[3], F f)
-{
-    s[0] = s[1] = s[2] = 0.0f;
-    if (i >= 0)
-        for (int e = __ldg(rs + i) + l; e < __ldg(rs + i + 1); e += G)
-        {
-            float g[3];
-            f(__ldg(cols + e), g);
-            const float v = __ldg(val + e);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) s[q] += v * g[q];
-        }
-#pragma unroll
-    for (int q = 0; q < 3; ++q)
-#pragma unroll
-        for (int o = G / 2; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-}
-
 struct Active3
 {
     bool a[3];
@@ -679,13 +420,11 @@ __device__ __forceinline__ Active3 active3(const int* done)
     return Active3{{done[0] == 0, done[1] == 0, done[2] == 0}};
 }
 
-// Level vectors of the three-component V-cycle, above the last level, hold
-// one float4 per row: the three components in x, y, z (w is zero).  A row
-// gathered by a neighbour's sweep or by its aggregate's restriction is one
-// 16-byte load, not three scattered ones.  The last level (the fused tail or
-// the dense coarsest solve) keeps component q at offset q * n, as the single
-// V-cycle's kernels there expect.  A converged component's lanes carry zeros
-// (its input lanes are read as zero), so every lane is computed and stored.
+// Level vectors of the three-component V-cycle hold one float4 per row: the
+// three components in x, y, z (w is zero).  A row gathered by a neighbour's
+// sweep or by its aggregate's restriction is one 16-byte load, not three
+// scattered ones.  A converged component's lanes carry zeros (its input lanes
+// are read as zero), so every lane is computed and stored.
 
 __device__ __forceinline__ float4 pack3(const float (&v)[3]) { return make_float4(v[0], v[1], v[2], 0.0f); }
 __device__ __forceinline__ void unpack3(float4 p, float (&v)[3])
@@ -728,151 +467,6 @@ __global__ void __launch_bounds__(TPB, (W > 0 && W <= 8) ? 6 : 1) k_amgv_pre0(co
     }
 }
 
-/// the residuals summed over each aggregate (a group of lanes per aggregate,
-/// lane l taking members l, l + G, ..., then the shuffle tree): the next
-/// level's right-hand side.  Into a level above the last one it also stores
-/// that level's first sweep w D^-1 b, which the level's residual pass
-/// gathers; into the last level it writes component q at offset q * nc.
-template <bool kLast, int G>
-__global__ void __launch_bounds__(TPB) k_amgv_restrict(const int* __restrict__ done, int nc, const int* __restrict__ ms,
-                                                       const int* __restrict__ mem, const float4* __restrict__ r,
-                                                       const float* __restrict__ dinvc, float4* __restrict__ bc,
-                                                       float4* __restrict__ xc, float* __restrict__ bcLast)
-{
-    pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    const int l = threadIdx.x % G;
-    const int stride = gridDim.x * (TPB / G);
-    for (int I0 = blockIdx.x * (TPB / G) + threadIdx.x / G;; I0 += stride)
-    {
-        const int base = I0 - (threadIdx.x % 32) / G;
-        if (base >= nc) break;
-        const int I = I0 < nc ? I0 : -1;
-        float s[3] = {0.0f, 0.0f, 0.0f};
-        if (I >= 0)
-            for (int k = __ldg(ms + I) + l; k < __ldg(ms + I + 1); k += G)
-            {
-                float v[3];
-                unpack3(__ldg(r + __ldg(mem + k)), v);
-#pragma unroll
-                for (int q = 0; q < 3; ++q) s[q] += v[q];
-            }
-#pragma unroll
-        for (int q = 0; q < 3; ++q)
-#pragma unroll
-            for (int o = G / 2; o > 0; o >>= 1) s[q] += __shfl_xor_sync(0xffffffffu, s[q], o);
-        if (I < 0 || l != 0) continue;
-        if constexpr (kLast)
-        {
-#pragma unroll
-            for (int q = 0; q < 3; ++q)
-                if (act.a[q]) bcLast[q * nc + I] = s[q];
-        }
-        else
-        {
-            const float wd = kOmega * dinvc[I];
-            float xv[3];
-#pragma unroll
-            for (int q = 0; q < 3; ++q) xv[q] = wd * s[q];
-            bc[I] = pack3(s);
-            xc[I] = pack3(xv);
-        }
-    }
-}
-
-/// coarse level, the residual of the first sweep: r = b - A x, with x the
-/// sweep the restriction into this level stored
-template <int G>
-__global__ void __launch_bounds__(TPB) k_amgv_pre(const int* __restrict__ done, int n, const int* __restrict__ rs,
-                                                  const int* __restrict__ cols, const float* __restrict__ val,
-                                                  const float4* __restrict__ x, const float4* __restrict__ b,
-                                                  float4* __restrict__ r)
-{
-    pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    const int l = threadIdx.x % G;
-    const int stride = gridDim.x * (TPB / G);
-    for (int i0 = blockIdx.x * (TPB / G) + threadIdx.x / G;; i0 += stride)
-    {
-        const int base = i0 - (threadIdx.x % 32) / G;
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        float s[3];
-        group_row3<G>(rs, cols, val, i, l, s, [&](int j, float (&g)[3]) { unpack3(__ldg(x + j), g); });
-        if (i >= 0 && l == 0)
-        {
-            float bi[3], rv[3];
-            unpack3(b[i], bi);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) rv[q] = bi[q] - s[q];
-            r[i] = pack3(rv);
-        }
-    }
-}
-
-/// the coarse corrections brought to this level: y = x + s P xc, with xc
-/// one float4 per row, or component q at offset q * nNext from the last level
-template <bool kFromLast>
-__global__ void __launch_bounds__(TPB) k_amgv_prolong(const int* __restrict__ done, int n, int nNext,
-                                                      const float4* __restrict__ x, const float4* __restrict__ xc,
-                                                      const float* __restrict__ xcLast, const int* __restrict__ agg,
-                                                      float4* __restrict__ y, float scale)
-{
-    pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    FOR_ROWS(i, n)
-    {
-        const int ai = agg[i];
-        float xv[3], cv[3], yv[3];
-        unpack3(x[i], xv);
-        if constexpr (kFromLast)
-        {
-#pragma unroll
-            for (int q = 0; q < 3; ++q) cv[q] = act.a[q] ? xcLast[q * nNext + ai] : 0.0f;
-        }
-        else
-            unpack3(xc[ai], cv);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) yv[q] = xv[q] + scale * cv[q];
-        y[i] = pack3(yv);
-    }
-}
-
-/// coarse level: xo = y + w D^-1 (b - A y)
-template <int G>
-__global__ void __launch_bounds__(TPB) k_amgv_post(const int* __restrict__ done, int n, const int* __restrict__ rs,
-                                                   const int* __restrict__ cols, const float* __restrict__ val,
-                                                   const float* __restrict__ dinv, const float4* __restrict__ b,
-                                                   const float4* __restrict__ y, float4* __restrict__ xo)
-{
-    pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    const int l = threadIdx.x % G;
-    const int stride = gridDim.x * (TPB / G);
-    for (int i0 = blockIdx.x * (TPB / G) + threadIdx.x / G;; i0 += stride)
-    {
-        const int base = i0 - (threadIdx.x % 32) / G;
-        if (base >= n) break;
-        const int i = i0 < n ? i0 : -1;
-        float s[3];
-        group_row3<G>(rs, cols, val, i, l, s, [&](int j, float (&g)[3]) { unpack3(__ldg(y + j), g); });
-        if (i >= 0 && l == 0)
-        {
-            const float di = dinv[i];
-            float bi[3], yi[3], xv[3];
-            unpack3(b[i], bi);
-            unpack3(y[i], yi);
-#pragma unroll
-            for (int q = 0; q < 3; ++q) xv[q] = yi[q] + kOmega * di * (bi[q] - s[q]);
-            xo[i] = pack3(xv);
-        }
-    }
-}
-
 /// finest level: z = y + w D^-1 (b - A y), into FP64 (active components only)
 template <int W>
 __global__ void __launch_bounds__(TPB) k_amgv_post0(const int* __restrict__ done, DMat A, const float* __restrict__ val,
@@ -897,9 +491,174 @@ __global__ void __launch_bounds__(TPB) k_amgv_post0(const int* __restrict__ done
     }
 }
 
-// ---- large coarse levels in SELL-32, one thread per row: the same
-// arithmetic as the lane-group passes, each row summed in its CSR column
-// order (the single and the three-vector V-cycle alike)
+// ---- the coarse levels, for one vector (V float) or three at once (V
+// float4, a component per lane of it): the same arithmetic and orders per
+// component, so the three-vector V-cycle gives each component the single
+// one's bits
+
+__device__ __forceinline__ void vzero(float& v) { v = 0.0f; }
+__device__ __forceinline__ void vzero(float4& v) { v = make_float4(0.0f, 0.0f, 0.0f, 0.0f); }
+__device__ __forceinline__ void vmad(float& s, float a, float v) { s += a * v; }
+__device__ __forceinline__ void vmad(float4& s, float a, float4 v)
+{
+    s.x += a * v.x;
+    s.y += a * v.y;
+    s.z += a * v.z;
+}
+__device__ __forceinline__ float vscaled(float a, float v) { return a * v; }
+__device__ __forceinline__ float4 vscaled(float a, float4 v) { return make_float4(a * v.x, a * v.y, a * v.z, 0.0f); }
+__device__ __forceinline__ float vadd(float a, float b) { return a + b; }
+__device__ __forceinline__ float4 vadd(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, 0.0f); }
+__device__ __forceinline__ float vsub(float a, float b) { return a - b; }
+__device__ __forceinline__ float4 vsub(float4 a, float4 b) { return make_float4(a.x - b.x, a.y - b.y, a.z - b.z, 0.0f); }
+template <int G>
+__device__ __forceinline__ void vgroup(float& s)
+{
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+}
+template <int G>
+__device__ __forceinline__ void vgroup(float4& s)
+{
+    vgroup<G>(s.x);
+    vgroup<G>(s.y);
+    vgroup<G>(s.z);
+}
+/// whether a kernel's vectors may still change: the single V-cycle's stop
+/// flag, or all three components' done flags
+__device__ __forceinline__ bool halted(const int* f, float) { return f && *f; }
+__device__ __forceinline__ bool halted(const int* f, float4) { return f[0] && f[1] && f[2]; }
+
+/// A coarse level on the device: its operator, its aggregates' members and
+/// its vectors (rhs, first sweep, residual, output).
+template <class V>
+struct Coarse
+{
+    int n;
+    const int *rs, *cols;
+    const float *val, *dinv;
+    const int *agg, *ms, *mem;  // to the next level
+    const int *sstart, *scol;   // SELL-32 copy (null: none)
+    const float* sval;
+    V *b, *x, *r, *o;
+    int gRow, gAgg;
+};
+
+/// Row i summed by a group of G lanes, lane l taking entries l, l + G, ...;
+/// the group's lanes hold the sum after the shuffle tree.
+template <class V, int G>
+__device__ __forceinline__ V group_row(const Coarse<V>& L, int i, int l, const V* x)
+{
+    V s;
+    vzero(s);
+    if (i >= 0)
+        for (int e = __ldg(L.rs + i) + l; e < __ldg(L.rs + i + 1); e += G)
+        {
+            const V* p = x + __ldg(L.cols + e);
+            vmad(s, __ldg(L.val + e), __ldg(p));
+        }
+    vgroup<G>(s);
+    return s;
+}
+
+/// Calls body(i, l) for every row in groups of G lanes; whole warps go round
+/// together (the shuffles need every lane), i is -1 past the last row.
+template <int G, class F>
+__device__ __forceinline__ void group_loop(int n, int thread, int threads, F&& body)
+{
+    const int l = threadIdx.x % G;
+    for (int i0 = thread / G;; i0 += threads / G)
+    {
+        if (i0 - (threadIdx.x % 32) / G >= n) break;
+        body(i0 < n ? i0 : -1, l);
+    }
+}
+
+/// the residual r of the level above summed over each of this level's n
+/// aggregates: its right-hand side b and, dinv given, first sweep x = w D^-1 b
+template <class V, int G>
+__device__ __forceinline__ void do_restrict(int n, const int* __restrict__ ms, const int* __restrict__ mem, const V* r,
+                                            const float* dinv, float w, V* b, V* x, int thread, int threads)
+{
+    group_loop<G>(n, thread, threads, [&](int I, int l) {
+        V s;
+        vzero(s);
+        if (I >= 0)
+            for (int k = __ldg(ms + I) + l; k < __ldg(ms + I + 1); k += G)
+            {
+                const V* p = r + __ldg(mem + k);
+                s = vadd(s, __ldg(p));
+            }
+        vgroup<G>(s);
+        if (I < 0 || l != 0) return;
+        b[I] = s;
+        if (dinv) x[I] = vscaled(w * dinv[I], s);
+    });
+}
+
+/// r = b - A x
+template <class V, int G>
+__device__ __forceinline__ void do_residual(const Coarse<V>& L, const V* x, V* r, int thread, int threads)
+{
+    group_loop<G>(L.n, thread, threads, [&](int i, int l) {
+        const V s = group_row<V, G>(L, i, l, x);
+        if (i >= 0 && l == 0) r[i] = vsub(L.b[i], s);
+    });
+}
+
+/// out = y + w D^-1 (b - A y)
+template <class V, int G>
+__device__ __forceinline__ void do_smooth(const Coarse<V>& L, float w, const V* y, V* out, int thread, int threads)
+{
+    group_loop<G>(L.n, thread, threads, [&](int i, int l) {
+        const V s = group_row<V, G>(L, i, l, y);
+        if (i >= 0 && l == 0) out[i] = vadd(y[i], vscaled(w * L.dinv[i], vsub(L.b[i], s)));
+    });
+}
+
+template <class V, int G>
+__global__ void __launch_bounds__(TPB) k_amg_restrict(const int* __restrict__ stop, int n, const int* __restrict__ ms,
+                                                      const int* __restrict__ mem, const V* __restrict__ r,
+                                                      const float* __restrict__ dinv, float w, V* __restrict__ b,
+                                                      V* __restrict__ x)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    do_restrict<V, G>(n, ms, mem, r, dinv, w, b, x, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+
+template <class V, int G>
+__global__ void __launch_bounds__(TPB) k_amg_residual(const int* __restrict__ stop, Coarse<V> L, const V* __restrict__ x,
+                                                      V* __restrict__ r)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    do_residual<V, G>(L, x, r, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+
+template <class V, int G>
+__global__ void __launch_bounds__(TPB) k_amg_smooth(const int* __restrict__ stop, Coarse<V> L, float w, const V* __restrict__ y,
+                                                    V* __restrict__ out)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    do_smooth<V, G>(L, w, y, out, blockIdx.x * TPB + threadIdx.x, gridDim.x * TPB);
+}
+
+/// the coarse correction brought to a level: y = x + s P xc
+template <class V>
+__global__ void __launch_bounds__(TPB) k_amg_prolong(const int* __restrict__ stop, int n, const V* __restrict__ x,
+                                                     const V* __restrict__ xc, const int* __restrict__ agg,
+                                                     V* __restrict__ y, float scale)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    FOR_ROWS(i, n) y[i] = vadd(x[i], vscaled(scale, xc[agg[i]]));
+}
+
+// Large coarse levels in SELL-32, one thread per row: each row summed in its
+// CSR column order; columns and values of eight slots are loaded before
+// their gathers.
 
 /// a coarse level's CSR values into its SELL-32 copy (the pads stay 0)
 __global__ void __launch_bounds__(TPB) k_amg_to_sell(int nnz, const int* __restrict__ pos, const float* __restrict__ val,
@@ -908,16 +667,12 @@ __global__ void __launch_bounds__(TPB) k_amg_to_sell(int nnz, const int* __restr
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < nnz; e += gridDim.x * blockDim.x) sval[pos[e]] = val[e];
 }
 
-/// row i of a SELL-32 operator: sum over its entries, slot by slot, of
-/// val * f(col) for NV values per column; columns and values of eight slots
-/// are loaded before their gathers
-template <int NV, class F>
-__device__ __forceinline__ void sell32_row(const int* __restrict__ sstart, const int* __restrict__ scol,
-                                           const float* __restrict__ sval, int i, float (&s)[NV], F f)
+template <class V>
+__device__ __forceinline__ V sell32_row(const Coarse<V>& L, int i, const V* __restrict__ x)
 {
-    const int e0 = __ldg(sstart + (i >> 5)) + (i & 31), e1 = __ldg(sstart + (i >> 5) + 1);
-#pragma unroll
-    for (int q = 0; q < NV; ++q) s[q] = 0.0f;
+    const int e0 = __ldg(L.sstart + (i >> 5)) + (i & 31), e1 = __ldg(L.sstart + (i >> 5) + 1);
+    V s;
+    vzero(s);
     for (int eb = e0; eb < e1; eb += 32 * 8)
     {
         int col[8];
@@ -926,102 +681,204 @@ __device__ __forceinline__ void sell32_row(const int* __restrict__ sstart, const
         for (int k = 0; k < 8; ++k)
         {
             const int e = eb + 32 * k;
-            col[k] = e < e1 ? __ldg(scol + e) : -1;
-            v[k] = e < e1 ? __ldg(sval + e) : 0.0f;
+            col[k] = e < e1 ? __ldg(L.scol + e) : -1;
+            v[k] = e < e1 ? __ldg(L.sval + e) : 0.0f;
         }
-        float g[8][NV];
+        V g[8];
 #pragma unroll
         for (int k = 0; k < 8; ++k)
         {
-            if (col[k] >= 0) f(col[k], g[k]);
-            else
-            {
-#pragma unroll
-                for (int q = 0; q < NV; ++q) g[k][q] = 0.0f;
-            }
+            if (col[k] >= 0) g[k] = __ldg(x + col[k]);
+            else vzero(g[k]);
         }
 #pragma unroll
-        for (int k = 0; k < 8; ++k)
+        for (int k = 0; k < 8; ++k) vmad(s, v[k], g[k]);
+    }
+    return s;
+}
+
+/// r = b - A x
+template <class V>
+__global__ void __launch_bounds__(TPB) k_amg_residual_sell(const int* __restrict__ stop, Coarse<V> L,
+                                                           const V* __restrict__ x, V* __restrict__ r)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    FOR_ROWS(i, L.n) r[i] = vsub(L.b[i], sell32_row(L, i, x));
+}
+
+/// out = y + w D^-1 (b - A y)
+template <class V>
+__global__ void __launch_bounds__(TPB) k_amg_smooth_sell(const int* __restrict__ stop, Coarse<V> L, float w,
+                                                         const V* __restrict__ y, V* __restrict__ out)
+{
+    pdl_entry();
+    if (halted(stop, V{})) return;
+    FOR_ROWS(i, L.n)
+    {
+        const V s = sell32_row(L, i, y);
+        out[i] = vadd(y[i], vscaled(w * L.dinv[i], vsub(L.b[i], s)));
+    }
+}
+
+// ---- the last levels ----------------------------------------------------------
+
+constexpr int kTailMax = 1024;  // rows of the fused last aggregation level
+constexpr int kTailThreads = 1024;
+constexpr int kTailLanes = 4;
+
+struct TailLevel
+{
+    int n, nc, nnz;
+    const int *rs, *cols, *agg, *ms, *mem;
+    const float *val, *dinv, *dense;
+    const float* b;  // this level's right-hand side and output: a vector's
+    float* o;        // values `stride` apart, vector q at offset q
+    int stride;
+    float scale;     // coarse-correction scaling
+    Sweeps w;
+};
+
+/// Shared-memory layout of k_amg_tail (4-byte words): the level's CSR
+/// (rs n + 1, cols nnz, val nnz), dinv n, agg n, the aggregates' member
+/// lists (ms nc + 1, mem n), the dense inverse nc * nc, the vectors b, x, r
+/// n each, bc and xc nc each.
+__host__ __device__ constexpr size_t tailSmemWords(int n, int nnz, int nc)
+{
+    return static_cast<size_t>(n + 1) + 2 * static_cast<size_t>(nnz) + 2 * static_cast<size_t>(n) +
+           static_cast<size_t>(nc + 1) + static_cast<size_t>(n) + static_cast<size_t>(nc) * nc + 3 * static_cast<size_t>(n) +
+           2 * static_cast<size_t>(nc);
+}
+
+/// The last aggregation level (at most kTailMax rows) and the coarsest solve
+/// in one block per vector, the level held in shared memory: one coalesced
+/// load of its matrix, aggregates, dense inverse and right-hand side, then
+/// the sweeps and the residual, restriction, dense solve, prolongation and
+/// the sweeps again, separated by block barriers.  Block q works on vector q
+/// and does nothing when done[q] is set (done may be null); only the output
+/// goes back to global memory.
+__global__ void __launch_bounds__(kTailThreads) k_amg_tail(const int* __restrict__ done, TailLevel T)
+{
+    pdl_entry();
+    const int q = blockIdx.x;
+    if (done && done[q]) return;
+    extern __shared__ __align__(16) int tsm[];
+    const int n = T.n, nc = T.nc, nnz = T.nnz, t = threadIdx.x;
+    int* rs = tsm;
+    int* cols = rs + (n + 1);
+    float* val = reinterpret_cast<float*>(cols + nnz);
+    float* dinv = val + nnz;
+    int* agg = reinterpret_cast<int*>(dinv + n);
+    int* ms = agg + n;
+    int* mem = ms + (nc + 1);
+    float* dense = reinterpret_cast<float*>(mem + n);
+    float* b = dense + static_cast<size_t>(nc) * nc;
+    float* x = b + n;
+    float* r = x + n;
+    float* bc = r + n;
+    float* xc = bc + nc;
+    for (int i = t; i <= n; i += kTailThreads) rs[i] = T.rs[i];
+    for (int e = t; e < nnz; e += kTailThreads)
+    {
+        cols[e] = T.cols[e];
+        val[e] = T.val[e];
+    }
+    for (int i = t; i < n; i += kTailThreads)
+    {
+        const float di = T.dinv[i], bi = T.b[static_cast<size_t>(i) * T.stride + q];
+        dinv[i] = di;
+        agg[i] = T.agg[i];
+        mem[i] = T.mem[i];
+        b[i] = bi;
+        x[i] = T.w.w[0] * di * bi;
+    }
+    for (int i = t; i <= nc; i += kTailThreads) ms[i] = T.ms[i];
+    for (int i = t; i < nc * nc; i += kTailThreads) dense[i] = T.dense[i];
+    __syncthreads();
+    const int l = t % kTailLanes, first = t / kTailLanes, stride = kTailThreads / kTailLanes;
+    // out(i, (A v)_i) for every row, a group of lanes per row
+    auto product = [&](const float* v, auto out) {
+        for (int i0 = first;; i0 += stride)
+        {
+            const int base = i0 - (t % 32) / kTailLanes;
+            if (base >= n) break;
+            const int i = i0 < n ? i0 : -1;
+            float s = 0.0f;
+            if (i >= 0)
+                for (int e = rs[i] + l; e < rs[i + 1]; e += kTailLanes) s += val[e] * v[cols[e]];
 #pragma unroll
-            for (int q = 0; q < NV; ++q) s[q] += v[k] * g[k][q];
-    }
-}
-
-/// single vector: x = w D^-1 b, r = b - A x
-__global__ void __launch_bounds__(TPB) k_amg_pre_sell(const int* __restrict__ stop, int n, const int* __restrict__ sstart,
-                                                      const int* __restrict__ scol, const float* __restrict__ sval,
-                                                      const float* __restrict__ dinv, const float* __restrict__ b,
-                                                      float* __restrict__ x, float* __restrict__ r)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    FOR_ROWS(i, n)
+            for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (i >= 0 && l == 0) out(i, s);
+        }
+        __syncthreads();
+    };
+    float *u = x, *v = r;
+    for (int k = 1; k < T.w.m; ++k)
     {
-        float s[1];
-        sell32_row<1>(sstart, scol, sval, i, s,
-                      [&](int j, float (&g)[1]) { g[0] = kOmega * __ldg(dinv + j) * __ldg(b + j); });
-        const float bi = b[i];
-        x[i] = kOmega * dinv[i] * bi;
-        r[i] = bi - s[0];
+        const float w = T.w.w[k];
+        product(u, [&](int i, float s) { v[i] = u[i] + w * dinv[i] * (b[i] - s); });
+        float* const c = u;
+        u = v;
+        v = c;
     }
-}
-
-/// single vector: xo = y + w D^-1 (b - A y)
-__global__ void __launch_bounds__(TPB) k_amg_post_sell(const int* __restrict__ stop, int n, const int* __restrict__ sstart,
-                                                       const int* __restrict__ scol, const float* __restrict__ sval,
-                                                       const float* __restrict__ dinv, const float* __restrict__ b,
-                                                       const float* __restrict__ y, float* __restrict__ xo)
-{
-    pdl_entry();
-    if (stop && *stop) return;
-    FOR_ROWS(i, n)
+    product(u, [&](int i, float s) { v[i] = b[i] - s; });
+    // restriction
+    for (int I0 = first;; I0 += stride)
     {
-        float s[1];
-        sell32_row<1>(sstart, scol, sval, i, s, [&](int j, float (&g)[1]) { g[0] = __ldg(y + j); });
-        xo[i] = y[i] + kOmega * dinv[i] * (b[i] - s[0]);
-    }
-}
-
-/// three vectors: r = b - A x, x the sweep the restriction stored
-__global__ void __launch_bounds__(TPB) k_amgv_pre_sell(const int* __restrict__ done, int n, const int* __restrict__ sstart,
-                                                       const int* __restrict__ scol, const float* __restrict__ sval,
-                                                       const float4* __restrict__ x, const float4* __restrict__ b,
-                                                       float4* __restrict__ r)
-{
-    pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    FOR_ROWS(i, n)
-    {
-        float s[3], bi[3], rv[3];
-        sell32_row<3>(sstart, scol, sval, i, s, [&](int j, float (&g)[3]) { unpack3(__ldg(x + j), g); });
-        unpack3(b[i], bi);
+        const int base = I0 - (t % 32) / kTailLanes;
+        if (base >= nc) break;
+        const int I = I0 < nc ? I0 : -1;
+        float s = 0.0f;
+        if (I >= 0)
+            for (int k = ms[I] + l; k < ms[I + 1]; k += kTailLanes) s += v[mem[k]];
 #pragma unroll
-        for (int q = 0; q < 3; ++q) rv[q] = bi[q] - s[q];
-        r[i] = pack3(rv);
+        for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (I >= 0 && l == 0) bc[I] = s;
     }
+    __syncthreads();
+    // the coarsest solve xc = M bc, a warp per row
+    {
+        const int lane = t & 31;
+        for (int i = t >> 5; i < nc; i += kTailThreads / 32)
+        {
+            float s = 0.0f;
+            for (int j = lane; j < nc; j += 32) s += dense[i * nc + j] * bc[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) xc[i] = s;
+        }
+    }
+    __syncthreads();
+    for (int i = t; i < n; i += kTailThreads) u[i] = u[i] + T.scale * xc[agg[i]];
+    __syncthreads();
+    for (int k = T.w.m - 1; k > 0; --k)
+    {
+        const float w = T.w.w[k];
+        product(u, [&](int i, float s) { v[i] = u[i] + w * dinv[i] * (b[i] - s); });
+        float* const c = u;
+        u = v;
+        v = c;
+    }
+    const float w = T.w.w[0];
+    product(u, [&](int i, float s) {
+        T.o[static_cast<size_t>(i) * T.stride + q] = u[i] + w * dinv[i] * (b[i] - s);
+    });
 }
 
-/// three vectors: xo = y + w D^-1 (b - A y)
-__global__ void __launch_bounds__(TPB) k_amgv_post_sell(const int* __restrict__ done, int n, const int* __restrict__ sstart,
-                                                        const int* __restrict__ scol, const float* __restrict__ sval,
-                                                        const float* __restrict__ dinv, const float4* __restrict__ b,
-                                                        const float4* __restrict__ y, float4* __restrict__ xo)
+/// the coarsest solve x = M b with the dense inverse, when the tail kernel
+/// does not hold the level above it (block q: vector q)
+__global__ void __launch_bounds__(kDenseMax) k_amg_dense(const int* __restrict__ done, int n, int stride,
+                                                         const float* __restrict__ m, const float* __restrict__ b,
+                                                         float* __restrict__ x)
 {
     pdl_entry();
-    const Active3 act = active3(done);
-    if (act.none()) return;
-    FOR_ROWS(i, n)
-    {
-        float s[3], bi[3], yi[3], xv[3];
-        sell32_row<3>(sstart, scol, sval, i, s, [&](int j, float (&g)[3]) { unpack3(__ldg(y + j), g); });
-        const float di = dinv[i];
-        unpack3(b[i], bi);
-        unpack3(y[i], yi);
-#pragma unroll
-        for (int q = 0; q < 3; ++q) xv[q] = yi[q] + kOmega * di * (bi[q] - s[q]);
-        xo[i] = pack3(xv);
-    }
+    const int q = blockIdx.x;
+    if (done && done[q]) return;
+    const int i = threadIdx.x;
+    if (i >= n) return;
+    float s = 0.0f;
+    for (int j = 0; j < n; ++j) s += m[i * n + j] * b[j * stride + q];
+    x[i * stride + q] = s;
 }
 
 /// a host CSR pattern whose entries remember where their values live
@@ -1087,8 +944,6 @@ std::vector<char> strongEntries(const Pattern& A, const std::vector<double>& v, 
 }
 
 }  // namespace
-
-static int tailLevel(const AmgState& a);
 
 /// A hierarchy's structure from the device matrix pattern (and, for
 /// strength of connection, the operator's values).
@@ -1285,7 +1140,7 @@ void Ctx::amgSetup(AmgUse use, const double* vals, double theta)
     }
     // the tail level's shared-memory copy, when it and the dense inverse fit
     // in one block's opt-in shared memory (set before any stream capture)
-    if (const int T = tailLevel(*a); T >= 0)
+    if (const int T = static_cast<int>(a->lv.size()) - 2; T >= 1 && a->lv[static_cast<size_t>(T)].n <= kTailMax)
     {
         const int nnz = a->lv[static_cast<size_t>(T) - 1].nnzNext;
         const size_t bytes = 4 * tailSmemWords(a->lv[T].n, nnz, a->lv[static_cast<size_t>(T) + 1].n);
@@ -1302,7 +1157,7 @@ void Ctx::amgSetup(AmgUse use, const double* vals, double theta)
                                    [&](const std::pair<int, size_t>& g) { return g.first == device_; });
             if (it == granted.end() || it->second < bytes)
             {
-                CFG_CUDA(cudaFuncSetAttribute(k_amg_tail_smem, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                CFG_CUDA(cudaFuncSetAttribute(k_amg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                               static_cast<int>(bytes)));
                 if (it == granted.end()) granted.push_back({device_, bytes});
                 else it->second = bytes;
@@ -1345,9 +1200,20 @@ void Ctx::amgValues(AmgUse use, const double* vals, const double* diag, const fl
     {
         const int n = a.nc;
         std::vector<float> v(a.hcols.size());
+        double theta = 0.0;
+        if (use == kAmgMomentum)
+        {
+            if (!a.skew) a.skew = alloc<double>(1);
+            CFG_CUDA(cudaMemsetAsync(a.skew, 0, sizeof(double), stream_));
+            k_amg_skew<<<GS_, TPB, 0, stream_>>>(DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals,
+                                                 reinterpret_cast<unsigned long long*>(a.skew));
+            launchCheck("amg_skew");
+            CFG_CUDA(cudaMemcpyAsync(&theta, a.skew, sizeof(double), cudaMemcpyDeviceToHost, stream_));
+        }
         if (!v.empty())
             CFG_CUDA(cudaMemcpyAsync(v.data(), a.lv.back().val, v.size() * sizeof(float), cudaMemcpyDeviceToHost, stream_));
         CFG_CUDA(cudaStreamSynchronize(stream_));
+        a.skewClass = skewOf(theta);
         std::vector<double> m(static_cast<size_t>(n) * n, 0.0), inv(static_cast<size_t>(n) * n, 0.0);
         double dmax = 0;
         for (int i = 0; i < n; ++i)
@@ -1405,195 +1271,238 @@ void Ctx::amgValues(AmgUse use, const double* vals, const double* diag, const fl
 /// post-smoothing also forms z.q and beta.
 void Ctx::amgApply(const double* r, double* z)
 {
-    amgCycle(r, z, nullptr, nullptr);
+    amgCycle(r, z, nullptr, nullptr, true);
+}
+
+namespace
+{
+template <class V>
+V* vecOf(float* one, float* three);
+template <>
+float* vecOf<float>(float* one, float*)
+{
+    return one;
+}
+template <>
+float4* vecOf<float4>(float*, float* three)
+{
+    return reinterpret_cast<float4*>(three);
+}
+
+template <class V>
+Coarse<V> coarseOf(const AmgLevel& L)
+{
+    Coarse<V> c{};
+    c.n = L.n;
+    c.rs = L.rs;
+    c.cols = L.cols;
+    c.val = L.val;
+    c.dinv = L.dinv;
+    c.agg = L.agg;
+    c.ms = L.ms;
+    c.mem = L.mem;
+    c.sstart = L.sstart;
+    c.scol = L.scol;
+    c.sval = L.sval;
+    c.b = vecOf<V>(L.b, L.b3);
+    c.x = vecOf<V>(L.x, L.x3);
+    c.r = vecOf<V>(L.r, L.r3);
+    c.o = vecOf<V>(L.xo, L.xo3);
+    c.gRow = L.gRow;
+    c.gAgg = L.gAgg;
+    return c;
+}
+
+/// The sweeps of the coarse levels in the solvers' V-cycles.  The plain
+/// aggregation hierarchy loses its contraction on the coarse levels, where
+/// sweeps cost a fraction of the finest level's; as Chebyshev polynomials over
+/// [lo, 1.9] (D^-1 A reaches 2 at most) two to four of them go further than
+/// damped Jacobi.  On the 2M-cell channel (B200, one outer iteration to
+/// 1e-12): one sweep 301 ms (1182 momentum component-iterations, 206 pressure
+/// iterations), two 178 ms (595, 131), three 170 ms (533, 101), four on the
+/// first coarse level and two below 159 ms (471, 106); four pay from
+/// kSellMinRows rows on, where a sweep is not a launch's latency
+/// (262k-cell channel 43 -> 32 ms with two, 29.5 with four; 158k-cell PISO
+/// step 10.6 -> 8.6 ms with two, 9.7 with four).  lo: 0.2 for two sweeps and
+/// 0.1 for four; convection narrows the choice (BiCGStab iterations of a
+/// numpy model, one sweep / four with lo 0.1 / with lo 0.3 / two damped
+/// Jacobi: theta 0.42 45/25/29/37, 0.71 63/57/49/61, 0.83 87/none/70/87, 0.88
+/// 110/none/90/107): class 1 takes lo 0.3, and only on large levels, where
+/// that is a gain over the launches it adds; class 2 keeps single sweeps.
+Smoother smootherOf(const AmgState& a)
+{
+    const bool large = a.lv.size() > 1 && a.lv[1].n >= kSellMinRows;
+    if (a.skewClass == 2 || (a.skewClass == 1 && !large)) return singleSweeps();
+    const double lo2 = a.skewClass == 1 ? 0.3 : 0.2, lo4 = a.skewClass == 1 ? 0.3 : 0.1;
+    return Smoother{large ? chebyshev(4, lo4, 1.9) : chebyshev(2, lo2, 1.9), chebyshev(2, lo2, 1.9)};
 }
 
 /// The level of the fused tail kernel (the last aggregated level, when it is
-/// not the finest and has at most kTailMax rows), or -1.
-static int tailLevel(const AmgState& a)
+/// not the finest and fits), or the dense level.
+int lastLevel(const AmgState& a)
 {
     const int L = static_cast<int>(a.lv.size());
-    return (L >= 3 && a.lv[L - 2].n <= kTailMax) ? L - 2 : -1;
+    return a.tailSmem ? L - 2 : L - 1;
 }
 
-/// The tail kernel's view of level T and the coarsest level: the single
-/// vectors (v3 false) or the three-vector ones.
-static TailLevel tailView(const AmgState& a, int T, bool v3, float scale)
+/// Everything of a V-cycle below the finest level: from the finest residual
+/// (level 0's r) to the finest level's corrected iterate (level 0's r, which
+/// the post-sweep reads).
+template <class V>
+void coarseCycle(const AmgState& a, bool pdl, int sms, cudaStream_t stream, const int* stop, float scale, const Smoother& sm)
 {
-    const AmgLevel& V = a.lv[static_cast<size_t>(T)];
-    const AmgLevel& C = a.lv[static_cast<size_t>(T) + 1];
-    TailLevel t{};
-    t.n = V.n;
-    t.nc = C.n;
-    t.rs = V.rs;
-    t.cols = V.cols;
-    t.agg = V.agg;
-    t.ms = V.ms;
-    t.mem = V.mem;
-    t.val = V.val;
-    t.dinv = V.dinv;
-    t.dense = a.dense;
-    t.b = v3 ? V.b3 : V.b;
-    t.x = v3 ? V.x3 : V.x;
-    t.r = v3 ? V.r3 : V.r;
-    t.y = t.r;  // the residual is restricted before the prolongation overwrites it
-    t.xo = v3 ? V.xo3 : V.xo;
-    t.bc = v3 ? C.b3 : C.b;
-    t.xc = v3 ? C.x3 : C.x;
-    t.scale = scale;
-    return t;
+    constexpr int vectors = sizeof(V) == sizeof(float) ? 1 : 3, stride = sizeof(V) / sizeof(float);
+    const int L = static_cast<int>(a.lv.size()), last = lastLevel(a);
+    auto grid = [&](int n) { return std::max(1, std::min((n + TPB - 1) / TPB, sms * 8)); };
+    // a group of G lanes per coarse row or aggregate
+    auto ggrid = [&](int n, int G) { return std::max(1, std::min((n + TPB / G - 1) / (TPB / G), sms * 8)); };
+    auto residual = [&](const Coarse<V>& C, const V* x, V* r) {
+        if (C.sstart)
+            launchK(pdl, k_amg_residual_sell<V>, waveGrid(reinterpret_cast<const void*>(k_amg_residual_sell<V>), sms, C.n),
+                    TPB, 0, stream, stop, C, x, r);
+        else
+            withGroup(C.gRow, [&](auto Gc) {
+                constexpr int G = decltype(Gc)::value;
+                launchK(pdl, k_amg_residual<V, G>, ggrid(C.n, G), TPB, 0, stream, stop, C, x, r);
+            });
+    };
+    auto smooth = [&](const Coarse<V>& C, float w, const V* y, V* out) {
+        if (C.sstart)
+            launchK(pdl, k_amg_smooth_sell<V>, waveGrid(reinterpret_cast<const void*>(k_amg_smooth_sell<V>), sms, C.n),
+                    TPB, 0, stream, stop, C, w, y, out);
+        else
+            withGroup(C.gRow, [&](auto Gc) {
+                constexpr int G = decltype(Gc)::value;
+                launchK(pdl, k_amg_smooth<V, G>, ggrid(C.n, G), TPB, 0, stream, stop, C, w, y, out);
+            });
+    };
+    for (int l = 0; l < last; ++l)
+    {
+        const Coarse<V> U = coarseOf<V>(a.lv[static_cast<size_t>(l)]), C = coarseOf<V>(a.lv[static_cast<size_t>(l) + 1]);
+        const bool inner = l + 1 < last;
+        const Sweeps& w = sm.at(l + 1);
+        withGroup(U.gAgg, [&](auto Gc) {
+            constexpr int G = decltype(Gc)::value;
+            launchK(pdl, k_amg_restrict<V, G>, ggrid(C.n, G), TPB, 0, stream, stop, C.n, U.ms, U.mem, U.r,
+                    inner ? C.dinv : static_cast<const float*>(nullptr), w.w[0], C.b, C.x);
+        });
+        if (!inner) break;
+        // x, o and r take turns; the iterate ends in x (an odd number of
+        // sweeps) or in o
+        V *x = C.x, *y = C.o;
+        for (int k = 1; k < w.m; ++k)
+        {
+            smooth(C, w.w[k], x, y);
+            std::swap(x, y);
+        }
+        residual(C, x, C.r);
+    }
+    const Coarse<V> B = coarseOf<V>(a.lv[static_cast<size_t>(last)]);
+    if (a.tailSmem)
+    {
+        TailLevel t{};
+        t.n = B.n;
+        t.nc = a.lv[static_cast<size_t>(last) + 1].n;
+        t.nnz = a.tailNnz;
+        t.rs = B.rs;
+        t.cols = B.cols;
+        t.agg = B.agg;
+        t.ms = B.ms;
+        t.mem = B.mem;
+        t.val = B.val;
+        t.dinv = B.dinv;
+        t.dense = a.dense;
+        t.b = reinterpret_cast<const float*>(B.b);
+        t.o = reinterpret_cast<float*>(B.o);
+        t.stride = stride;
+        t.scale = scale;
+        t.w = sm.at(last);
+        launchK(pdl, k_amg_tail, vectors, kTailThreads, a.tailSmem, stream, stop, t);
+    }
+    else
+        launchK(pdl, k_amg_dense, vectors, kDenseMax, 0, stream, stop, a.nc, stride, a.dense,
+                reinterpret_cast<const float*>(B.b), reinterpret_cast<float*>(B.x));
+    for (int l = last - 1; l >= 0; --l)
+    {
+        const Coarse<V> C = coarseOf<V>(a.lv[static_cast<size_t>(l)]), N = coarseOf<V>(a.lv[static_cast<size_t>(l) + 1]);
+        const Sweeps& w = sm.at(l);
+        const bool odd = l == 0 || (w.m & 1);
+        V *y = odd ? C.r : C.x, *t = odd ? C.o : C.r;
+        launchK(pdl, k_amg_prolong<V>, grid(C.n), TPB, 0, stream, stop, C.n, odd ? C.x : C.o, l + 1 == L - 1 ? N.x : N.o,
+                C.agg, y, scale);
+        if (l == 0) break;
+        // sweeps through the two free vectors in reverse, the last into o
+        for (int k = w.m - 1; k > 0; --k)
+        {
+            smooth(C, w.w[k], y, t);
+            std::swap(y, t);
+        }
+        smooth(C, w.w[0], y, C.o);
+    }
 }
 
-void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st)
+/// the kernels of coarseCycle
+int coarseKernels(const AmgState& a, const Smoother& sm)
+{
+    int k = 2;
+    for (int l = 1; l < lastLevel(a); ++l) k += 2 + 2 * sm.at(l).m;
+    return k + 1;
+}
+}  // namespace
+
+void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single)
 {
     if (!amg_) fail(CFG_EINVAL, "amg: the hierarchy is not set up (amgValues)");
     AmgState& a = *amg_;
     if (!a.valuesReady) fail(CFG_EINVAL, "amg: values not set up");
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
-    const int L = static_cast<int>(a.lv.size());
-    const int T = tailLevel(a);
-    const int last = T >= 0 ? T : L - 1;  // levels [0, last) run level by level
     const int* stop = st ? &st->done : nullptr;
-    auto grid = [&](int n) { return std::max(1, std::min((n + TPB - 1) / TPB, sms_ * 8)); };
-    // a group of G lanes per coarse row or aggregate
-    auto ggrid = [&](int n, int G) { return std::max(1, std::min((n + TPB / G - 1) / (TPB / G), sms_ * 8)); };
     const int Wsel = maxW_ <= 7 ? 7 : (maxW_ <= 16 ? 16 : 0);
-    // down
-    for (int l = 0; l < last; ++l)
-    {
-        AmgLevel& V = a.lv[l];
-        AmgLevel& N = a.lv[l + 1];
-        if (l == 0)
-        {
-            const auto pre0 = Wsel == 7 ? k_amg_pre0<7> : (Wsel == 16 ? k_amg_pre0<16> : k_amg_pre0<0>);
-            launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_,
-                stop, A, a.vals32, V.dinv, r, V.x, V.r);
-        }
-        else if (V.sstart)
-            launchK(pdl_, k_amg_pre_sell, waveGrid(reinterpret_cast<const void*>(k_amg_pre_sell), sms_, V.n), TPB, 0,
-                    stream_, stop, V.n, V.sstart, V.scol, V.sval, V.dinv, V.b, V.x, V.r);
-        else
-            withGroup(V.gRow, [&](auto Gc) {
-                constexpr int G = decltype(Gc)::value;
-                launchK(pdl_, k_amg_pre<G>, ggrid(V.n, G), TPB, 0, stream_, stop, V.n, V.rs, V.cols, V.val, V.dinv, V.b, V.x, V.r);
-            });
-        withGroup(V.gAgg, [&](auto Gc) {
-            constexpr int G = decltype(Gc)::value;
-            launchK(pdl_, k_amg_restrict<G>, ggrid(N.n, G), TPB, 0, stream_, stop, N.n, V.ms, V.mem, V.r, N.b);
-        });
-    }
-    if (T >= 0 && a.tailSmem)
-        launchK(pdl_, k_amg_tail_smem, 1, kTailThreads, a.tailSmem, stream_, stop, tailView(a, T, false, kScale), a.tailNnz);
-    else if (T >= 0) launchK(pdl_, k_amg_tail, 1, kTailThreads, 0, stream_, stop, tailView(a, T, false, kScale));
-    else launchK(pdl_, k_amg_dense, 1, kDenseMax, 0, stream_, stop, a.nc, a.dense, a.lv[L - 1].b, a.lv[L - 1].x);
-    // up: each level corrects with the next level's output
-    for (int l = last - 1; l >= 0; --l)
-    {
-        AmgLevel& V = a.lv[l];
-        const AmgLevel& N = a.lv[l + 1];
-        const float* xc = (l + 1 == L - 1) ? N.x : N.xo;
-        launchK(pdl_, k_amg_prolong, grid(V.n), TPB, 0, stream_, stop, V.n, V.x, xc, V.agg, V.r);
-        if (l == 0)
-        {
-            // one block partial per block: the grid is at most G_ blocks,
-            // which partials_ holds
-            const auto post0 = Wsel == 7 ? k_amg_post0<7> : (Wsel == 16 ? k_amg_post0<16> : k_amg_post0<0>);
-            launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_,
-                stop, A, a.vals32, V.dinv, r, V.r, z, q, partials_, st);
-        }
-        else if (V.sstart)
-            launchK(pdl_, k_amg_post_sell, waveGrid(reinterpret_cast<const void*>(k_amg_post_sell), sms_, V.n), TPB, 0,
-                    stream_, stop, V.n, V.sstart, V.scol, V.sval, V.dinv, V.b, V.r, V.xo);
-        else
-            withGroup(V.gRow, [&](auto Gc) {
-                constexpr int G = decltype(Gc)::value;
-                launchK(pdl_, k_amg_post<G>, ggrid(V.n, G), TPB, 0, stream_, stop, V.n, V.rs, V.cols, V.val, V.dinv, V.b, V.r, V.xo);
-            });
-    }
-    launchCheck("amg_vcycle", amgCycleKernels());
+    const AmgLevel& V = a.lv[0];
+    const auto pre0 = Wsel == 7 ? k_amg_pre0<7> : (Wsel == 16 ? k_amg_pre0<16> : k_amg_pre0<0>);
+    launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32, V.dinv,
+            r, V.x, V.r);
+    const Smoother sm = single ? singleSweeps() : smootherOf(a);
+    coarseCycle<float>(a, pdl_, sms_, stream_, stop, kScale, sm);
+    // one block partial per block: the grid is at most G_ blocks, which
+    // partials_ holds
+    const auto post0 = Wsel == 7 ? k_amg_post0<7> : (Wsel == 16 ? k_amg_post0<16> : k_amg_post0<0>);
+    launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
+            V.dinv, r, V.r, z, q, partials_, st);
+    launchCheck("amg_vcycle", amgCycleKernels(kAmgPressure, single));
 }
 
 /// z_q = V-cycle(b_q) for the three components whose done flag is clear
 /// (the BiCGStab's flags; a converged component keeps its old z_q)
-void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, const std::function<void(int)>& mark)
+void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, bool single,
+                    const std::function<void(int)>& mark)
 {
     if (!amgSlot(use)) fail(CFG_EINVAL, "amg: the hierarchy is not set up (amgValues)");
     AmgState& a = *amgSlot(use);
     if (!a.valuesReady) fail(CFG_EINVAL, "amg: values not set up");
     if (!a.lv[0].x3) fail(CFG_EINVAL, "amg: the three-component vectors are not allocated (amgVectors3)");
-    const int L = static_cast<int>(a.lv.size());
-    const int T = tailLevel(a);
-    const int last = T >= 0 ? T : L - 1;
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
-    auto grid = [&](int n) { return std::max(1, std::min((n + TPB - 1) / TPB, sms_ * 8)); };
-    auto ggrid = [&](int n, int G) { return std::max(1, std::min((n + TPB / G - 1) / (TPB / G), sms_ * 8)); };
     const int Wsel = maxW_ <= 7 ? 7 : (maxW_ <= 16 ? 16 : 0);
-    // levels above `last` hold a float4 per row; `last` (the tail level or
-    // the dense coarsest) holds component q at q * n
-    auto f4 = [](float* p) { return reinterpret_cast<float4*>(p); };
-    for (int l = 0; l < last; ++l)
-    {
-        AmgLevel& V = a.lv[l];
-        AmgLevel& N = a.lv[l + 1];
-        if (l == 0)
-        {
-            const auto pre0 = Wsel == 7 ? k_amgv_pre0<7> : (Wsel == 16 ? k_amgv_pre0<16> : k_amgv_pre0<0>);
-            launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_,
-                done, A, a.vals32, V.dinv, b, f4(V.x3), f4(V.r3));
-            if (mark) mark(0);
-        }
-        else if (V.sstart)
-            launchK(pdl_, k_amgv_pre_sell, waveGrid(reinterpret_cast<const void*>(k_amgv_pre_sell), sms_, V.n), TPB, 0,
-                    stream_, done, V.n, V.sstart, V.scol, V.sval, f4(V.x3), f4(V.b3), f4(V.r3));
-        else
-            withGroup(V.gRow, [&](auto Gc) {
-                constexpr int G = decltype(Gc)::value;
-                launchK(pdl_, k_amgv_pre<G>, ggrid(V.n, G), TPB, 0, stream_, done, V.n, V.rs, V.cols, V.val, f4(V.x3), f4(V.b3),
-                                                                  f4(V.r3));
-            });
-        withGroup(V.gAgg, [&](auto Gc) {
-            constexpr int G = decltype(Gc)::value;
-            if (l + 1 == last)
-                launchK(pdl_, k_amgv_restrict<true, G>, ggrid(N.n, G), TPB, 0, stream_, done, N.n, V.ms, V.mem, f4(V.r3), nullptr,
-                                                                             nullptr, nullptr, N.b3);
-            else
-                launchK(pdl_, k_amgv_restrict<false, G>, ggrid(N.n, G), TPB, 0, stream_, done, N.n, V.ms, V.mem, f4(V.r3), N.dinv,
-                                                                              f4(N.b3), f4(N.x3), nullptr);
-        });
-    }
-    if (T >= 0 && a.tailSmem)
-        launchK(pdl_, k_amg_tail_smem, 3, kTailThreads, a.tailSmem, stream_, done, tailView(a, T, true, scale), a.tailNnz);
-    else if (T >= 0) launchK(pdl_, k_amg_tail, 3, kTailThreads, 0, stream_, done, tailView(a, T, true, scale));
-    else launchK(pdl_, k_amg_dense, 3, kDenseMax, 0, stream_, done, a.nc, a.dense, a.lv[L - 1].b3, a.lv[L - 1].x3);
-    for (int l = last - 1; l >= 0; --l)
-    {
-        AmgLevel& V = a.lv[l];
-        const AmgLevel& N = a.lv[l + 1];
-        if (l + 1 == last)
-            launchK(pdl_, k_amgv_prolong<true>, grid(V.n), TPB, 0, stream_, done, V.n, N.n, f4(V.x3), nullptr,
-                                                                 (l + 1 == L - 1) ? N.x3 : N.xo3, V.agg, f4(V.r3),
-                                                                 scale);
-        else
-            launchK(pdl_, k_amgv_prolong<false>, grid(V.n), TPB, 0, stream_, done, V.n, N.n, f4(V.x3), f4(N.xo3), nullptr, V.agg,
-                                                                  f4(V.r3), scale);
-        if (l == 0)
-        {
-            if (mark) mark(1);
-            const auto post0 = Wsel == 7 ? k_amgv_post0<7> : (Wsel == 16 ? k_amgv_post0<16> : k_amgv_post0<0>);
-            launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_,
-                done, A, a.vals32, V.dinv, b, f4(V.r3), z);
-        }
-        else if (V.sstart)
-            launchK(pdl_, k_amgv_post_sell, waveGrid(reinterpret_cast<const void*>(k_amgv_post_sell), sms_, V.n), TPB, 0,
-                    stream_, done, V.n, V.sstart, V.scol, V.sval, V.dinv, f4(V.b3), f4(V.r3), f4(V.xo3));
-        else
-            withGroup(V.gRow, [&](auto Gc) {
-                constexpr int G = decltype(Gc)::value;
-                launchK(pdl_, k_amgv_post<G>, ggrid(V.n, G), TPB, 0, stream_, done, V.n, V.rs, V.cols, V.val, V.dinv, f4(V.b3),
-                                                                   f4(V.r3), f4(V.xo3));
-            });
-    }
-    launchCheck("amg_vcycle3", amgCycleKernels(use));
+    const AmgLevel& V = a.lv[0];
+    float4* const x = reinterpret_cast<float4*>(V.x3);
+    float4* const r = reinterpret_cast<float4*>(V.r3);
+    const auto pre0 = Wsel == 7 ? k_amgv_pre0<7> : (Wsel == 16 ? k_amgv_pre0<16> : k_amgv_pre0<0>);
+    launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32, V.dinv,
+            b, x, r);
+    if (mark) mark(0);
+    coarseCycle<float4>(a, pdl_, sms_, stream_, done, scale, single ? singleSweeps() : smootherOf(a));
+    if (mark) mark(1);
+    const auto post0 = Wsel == 7 ? k_amgv_post0<7> : (Wsel == 16 ? k_amgv_post0<16> : k_amgv_post0<0>);
+    launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32,
+            V.dinv, b, r, z);
+    launchCheck("amg_vcycle3", amgCycleKernels(use, single));
+}
+
+/// what the captured V-cycles of a hierarchy depend on beyond its pointers
+int Ctx::amgVariant(AmgUse use) const
+{
+    const AmgState* a = use == kAmgMomentum ? amgU_.get() : amg_.get();
+    return a ? a->skewClass : 0;
 }
 
 void Ctx::setAmgStrength(double theta)
@@ -1613,7 +1522,7 @@ void Ctx::amgVectors3(AmgUse use)
     for (auto& V : amgSlot(use)->lv)
         if (!V.x3)
         {
-            const size_t m = 4 * static_cast<size_t>(V.n);  // a float4 per row, or three rows of n
+            const size_t m = 4 * static_cast<size_t>(V.n);  // a float4 per row
             V.b3 = alloc<float>(m);
             V.x3 = alloc<float>(m);
             V.r3 = alloc<float>(m);
@@ -1621,14 +1530,11 @@ void Ctx::amgVectors3(AmgUse use)
         }
 }
 
-/// The number of kernels one amgCycle3 launches.
-int Ctx::amgCycleKernels(AmgUse use) const
+/// The number of kernels one V-cycle launches.
+int Ctx::amgCycleKernels(AmgUse use, bool single) const
 {
     const AmgState* a = use == kAmgMomentum ? amgU_.get() : amg_.get();
-    if (!a) return 0;
-    const int T = tailLevel(*a);
-    const int last = T >= 0 ? T : static_cast<int>(a->lv.size()) - 1;
-    return 4 * last + 1;
+    return a ? 2 + coarseKernels(*a, single ? singleSweeps() : smootherOf(*a)) : 0;
 }
 
 namespace
@@ -1822,7 +1728,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     else if (Wsel == 16) spmvInit(std::integral_constant<int, 16>{});
     else spmvInit(std::integral_constant<int, 0>{});
     launchCheck("fcgd_init");
-    amgCycle(r, z, nullptr, a.st);
+    amgCycle(r, z, nullptr, a.st, false);
     launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, p, a.st, 1);
     launchCheck("fcgd_p0");
     const auto spmv = Wsel == 7 ? k_fcgd_spmv<7> : (Wsel == 16 ? k_fcgd_spmv<16> : k_fcgd_spmv<0>);
@@ -1830,7 +1736,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     auto iteration = [&]() {
         launchK(pdl_, spmv, spmvGrid, TPB, 0, stream_, A, vals, p, r, q, partials_, a.st);
         launchK(pdl_, k_fcgd_update, GS_, TPB, 0, stream_, n, p, q, x, r, partials_, a.st);
-        amgCycle(r, z, q, a.st);
+        amgCycle(r, z, q, a.st, false);
         launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, p, a.st, 0);
         launchCheck("fcgd_iter", 3);
     };
@@ -1860,7 +1766,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
         if (ge) CFG_CUDA(cudaGraphLaunch(ge, stream_));
         else
             for (int k = 0; k < m; ++k) iteration();
-        launches_ = counted + static_cast<int64_t>(m) * (3 + amgCycleKernels());
+        launches_ = counted + static_cast<int64_t>(m) * (3 + amgCycleKernels(kAmgPressure, false));
         launched += m;
         chunk = std::min(chunk * 2, 32);
     }

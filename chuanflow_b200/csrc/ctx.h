@@ -294,12 +294,16 @@ private:
     void amgSetup(AmgUse use, const double* vals, double theta);
     void amgValues(AmgUse use, const double* vals, const double* diag, const float* vals32);
     void amgApply(const double* r, double* z);
-    void amgCycle(const double* r, double* z, const double* q, FcgState* st);
+    /// single: one sweep before and after each correction on every level, else
+    /// the hierarchy's own smoothers on the coarse ones
+    void amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single);
     /// mark(0) after the finest pre-sweep, mark(1) before the finest
     /// post-sweep (kernel timing), when given
-    void amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, const std::function<void(int)>& mark = {});
+    void amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, bool single,
+                   const std::function<void(int)>& mark = {});
     void amgVectors3(AmgUse use);
-    int amgCycleKernels(AmgUse use = kAmgPressure) const;
+    int amgCycleKernels(AmgUse use, bool single) const;
+    int amgVariant(AmgUse use) const;
     void amgFcg(const double* vals, const double* b, double* x, double tol, int maxIter, int normType,
                 cfg_solver_report* rep);
     void amgInfo(double* out);

@@ -1615,7 +1615,7 @@ void Ctx::teamReport(int nComp, cfg_solver_report* reps)
 void Ctx::checkTeam() const
 {
     if (*static_cast<volatile int*>(teamFailed_))
-        fail(CFG_ECUDA, "solver: a grid barrier's wait ran out");
+        fail(CFG_ECUDA, "solver: a wait inside a kernel ran out");
 }
 
 void Ctx::runCG(const double* vals, const double* diag, const double* b, double* x, double tol, int maxIter,
@@ -1817,7 +1817,7 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
     init.nComp = 3;
     const int n = dm_.nC;
     const int* done = reinterpret_cast<const int*>(reinterpret_cast<const char*>(st_) + offsetof(SolveState, done));
-    const int vk = amgCycleKernels(kAmgMomentum);
+    const int vk = amgCycleKernels(kAmgMomentum, false);
     CFG_CUDA(cudaMemcpyAsync(st_, &init, sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     auto loop = [&](auto Wc) {
         constexpr int W = decltype(Wc)::value;
@@ -1845,19 +1845,21 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
             for (int q = 0; q < 3; ++q) activeBefore += stHost_->done[q] ? 0 : 1;
             if (stHost_->allDone || launched >= maxIter) break;
             const int m = ktime_ ? 1 : std::min(chunk, maxIter - launched);
-            launchChunk(ptrKey("bicga", {vals, diag, x.c[0], x.c[1], x.c[2]}, W), m, [&](int k) {
+            launchChunk(ptrKey("bicga", {vals, diag, x.c[0], x.c[1], x.c[2]}, W * 4 + amgVariant(kAmgMomentum)), m, [&](int k) {
                 const std::function<void(int)> markZ = [&](int j) { tmark(k, 2 + j); };
                 const std::function<void(int)> markS = [&](int j) { tmark(k, 7 + j); };
                 tmark(k, 0);
                 launchK(pdl_, k_bia_p<3>, GS_, TPB, 0, stream_, n, br_, bp_, bv_, st_);
                 tmark(k, 1);
-                amgCycle3(kAmgMomentum, cv(bp_), bz_, done, kAmgScaleMomentum, ktime_ ? markZ : std::function<void(int)>{});
+                amgCycle3(kAmgMomentum, cv(bp_), bz_, done, kAmgScaleMomentum, false,
+                          ktime_ ? markZ : std::function<void(int)>{});
                 tmark(k, 4);
                 launchK(pdl_, k_bi_spmv1<W, 3>, GS_, TPB, 0, stream_, A, vals, bz_, bv_, br0_, partials_, st_);
                 tmark(k, 5);
                 launchK(pdl_, k_bia_s<3>, GS_, TPB, 0, stream_, n, br_, bv_, bs_, st_);
                 tmark(k, 6);
-                amgCycle3(kAmgMomentum, cv(bs_), bsh_, done, kAmgScaleMomentum, ktime_ ? markS : std::function<void(int)>{});
+                amgCycle3(kAmgMomentum, cv(bs_), bsh_, done, kAmgScaleMomentum, false,
+                          ktime_ ? markS : std::function<void(int)>{});
                 tmark(k, 9);
                 launchK(pdl_, k_bia_spmv2<W, 3>, GS_, TPB, 0, stream_, A, vals, bsh_, bs_, bt_, partials_, st_);
                 tmark(k, 10);
@@ -1872,6 +1874,7 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
         }
     };
     dispatchW(maxW_, [&](auto Wc) { loop(Wc); });
+    checkTeam();
     for (int q = 0; q < 3; ++q)
     {
         reps[q].iterations = stHost_->it[q];
@@ -3011,7 +3014,7 @@ void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3])
     // the pressure V-cycle's coarse-correction scale, so that each component
     // equals the single V-cycle's result
     amgCycle3(kAmgPressure, cv(bp_), bz_, reinterpret_cast<const int*>(reinterpret_cast<const char*>(st_) + offsetof(SolveState, done)),
-              kAmgScalePressure);
+              kAmgScalePressure, true);
     for (int q = 0; q < 3; ++q) fromDevCells(z + static_cast<size_t>(q) * dm_.nC, bz_.c[q], 1, 0);
 }
 
