@@ -16,6 +16,19 @@
 namespace cfg
 {
 
+/// The team of blocks a whole Krylov solve runs in as one kernel
+/// (persist.cuh): no team (blocks 0: the per-iteration kernels), a cluster or
+/// a cooperative grid per NC components, rows per thread and rows per block.
+struct TeamPlan
+{
+    int blocks = 0;  // per team
+    bool cluster = false;
+    int NC = 1;      // components per team
+    int K = 0, chunk = 0;
+};
+TeamPlan teamPlanOf(int n, int nComp, int clusterMax, int sms, bool gridOk);
+int largestCluster(int device);
+
 struct Timing
 {
     cudaEvent_t ev[16];
@@ -199,16 +212,6 @@ private:
     int uPrecond_ = CFG_PRECOND_JACOBI;
     float* uVal32_ = nullptr;
     void launchCheck(const char* what, int kernels = 1);
-    /// The team of blocks a whole Krylov solve runs in as one kernel
-    /// (persist.cuh): no team (blocks 0: the per-iteration kernels), a
-    /// cluster or a cooperative grid, rows per thread and rows per block.
-    struct TeamPlan
-    {
-        int blocks = 0;  // per team
-        bool cluster = false;
-        int NC = 1;      // components per team
-        int K = 0, chunk = 0;
-    };
     TeamPlan teamPlan(int nComp, bool bicg) const;
     template <class Kern, class A>
     void teamLaunch(const TeamPlan& tp, int teams, Kern kernel, const A& args, size_t smem, double tol, int maxIter, int normType);

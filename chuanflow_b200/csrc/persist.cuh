@@ -18,6 +18,45 @@ namespace cfg
 /// the diagonal), tetrahedra and prisms fit
 constexpr int kResW = 7;
 
+/// The matrix of a resident solve: row c's entries in order, e = first(c),
+/// first(c) + step, ... while live(e, c); its diagonal as the solvers take it.
+struct SellView
+{
+    DMat A;
+    const double* val;
+    const double* diag_;
+    static constexpr int step = 32;
+    static constexpr bool checked = false;  // rows are known to fit kResW
+    __device__ __forceinline__ int n() const { return A.n; }
+    __device__ __forceinline__ long long first(int c) const { return __ldg(A.start + (c >> 5)) + (c & 31); }
+    __device__ __forceinline__ long long end(int c) const { return __ldg(A.start + (c >> 5) + 1); }
+    __device__ __forceinline__ int col(long long e) const { return __ldg(A.col + e); }
+    __device__ __forceinline__ double value(long long e) const { return __ldg(val + e); }
+    __device__ __forceinline__ double diag(int c) const { return __ldg(diag_ + c); }
+};
+/// A caller's CSR with 32- or 64-bit indices, as it is.
+template <class I>
+struct CsrView
+{
+    int rows;
+    const I *rs, *cols;
+    const double* val;
+    static constexpr int step = 1;
+    static constexpr bool checked = true;
+    __device__ __forceinline__ int n() const { return rows; }
+    __device__ __forceinline__ long long first(int c) const { return __ldg(rs + c); }
+    __device__ __forceinline__ long long end(int c) const { return __ldg(rs + c + 1); }
+    __device__ __forceinline__ int col(long long e) const { return static_cast<int>(__ldg(cols + e)); }
+    __device__ __forceinline__ double value(long long e) const { return __ldg(val + e); }
+    /// the first entry in the diagonal column, else 0 (SparseMatrix::diagonal)
+    __device__ __forceinline__ double diag(int c) const
+    {
+        for (long long e = first(c); e < end(c); ++e)
+            if (col(e) == c) return value(e);
+        return 0.0;
+    }
+};
+
 /// A solve's arguments beyond its vectors: the stopping test, the rows per
 /// block (contiguous), where the outcome goes, and the optional
 /// {iterations, unconverged} sums of an outer iteration.
@@ -76,24 +115,25 @@ struct Resident
     }
     /// the block's entries from the SELL rows; slots past the last row and
     /// past a row's last entry are zero values at slot 0
-    __device__ __forceinline__ void load(const DMat& A, const double* __restrict__ v, int chunk, int rank)
+    template <class Mat>
+    __device__ __forceinline__ void load(const Mat& A, int chunk, int rank)
     {
         const unsigned base = static_cast<unsigned>(__cvta_generic_to_shared(buf));
 #pragma unroll
         for (int s = 0; s < K; ++s)
         {
             const int i = threadIdx.x + s * kTeamThreads, c = lo + i;
-            int e0 = 0, e1 = 0;
+            long long e0 = 0, e1 = 0;
             if (i < cnt)
             {
-                e0 = __ldg(A.start + (c >> 5)) + (c & 31);
-                e1 = __ldg(A.start + (c >> 5) + 1);
+                e0 = A.first(c);
+                e1 = A.end(c);
             }
 #pragma unroll
             for (int k = 0; k < kResW; ++k)
             {
-                const int e = e0 + 32 * k;
-                const int col = e < e1 ? __ldg(A.col + e) : -1;
+                const long long e = e0 + Mat::step * k;
+                const int col = e < e1 ? A.col(e) : -1;
                 int cd = 0;
                 if (col >= 0)
                 {
@@ -109,7 +149,7 @@ struct Resident
                     }
                     else cd = ~col;
                 }
-                const double ve = col >= 0 ? __ldg(v + e) : 0.0;
+                const double ve = col >= 0 ? A.value(e) : 0.0;
                 if constexpr (kRegs)
                 {
                     rv[s][k] = ve;
@@ -186,11 +226,10 @@ struct Resident
     }
 };
 
+template <class Mat>
 struct PersCg
 {
-    DMat A;
-    const double* val;
-    const double* diag;
+    Mat A;
     const double* b;
     double* x;
     double* g;  // a grid team's copy of the gather vector
@@ -247,19 +286,19 @@ __device__ __forceinline__ void pers_dic(Team& tm, Res& R, int C, const double (
 struct CgScalars
 {
     double alpha, beta;
-    int go;
+    int go, fits;
 };
 
 /// CG of Matrix.cpp:153-222, preconditioned by D^-1 or the multicolour DIC
-template <int K, class Team, bool kDic>
-__global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs t)
+template <int K, class Team, bool kDic, class Mat>
+__global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, PersArgs t)
 {
     __shared__ TeamSmem smem;
     extern __shared__ __align__(16) unsigned char dyn[];
     Team tm(smem, t.g);
-    const int n = a.A.n, lo = min(n, tm.rank * t.chunk), cnt = min(n - lo, t.chunk);
+    const int n = a.A.n(), lo = min(n, tm.rank * t.chunk), cnt = min(n - lo, t.chunk);
     Resident<K, 1, Team, resident_regs(K, 1, !kDic)> R(dyn, V3P{{a.g, a.g, a.g}}, lo, cnt);
-    R.load(a.A, a.val, t.chunk, tm.rank);
+    R.load(a.A, t.chunk, tm.rank);
     const bool two = t.normType != 0;
     __shared__ CgScalars sc;
     unsigned long long none[1] = {0};
@@ -282,10 +321,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
             {
                 const int c = lo + i;
                 col[k] = __ldg(a.colour + c);
-                const int e0 = __ldg(a.A.start + (c >> 5)) + (c & 31), e1 = __ldg(a.A.start + (c >> 5) + 1);
-                for (int j = 0; j < kResW && e0 + 32 * j < e1; ++j)
+                const long long e0 = a.A.first(c), e1 = a.A.end(c);
+                for (int j = 0; j < kResW && e0 + Mat::step * j < e1; ++j)
                 {
-                    const int cj = __ldg(a.A.col + e0 + 32 * j);
+                    const int cj = a.A.col(e0 + Mat::step * j);
                     if (cj < 0) break;
                     const int oc = __ldg(a.colour + cj);
                     if (oc < col[k]) lower[k] |= 1u << j;
@@ -293,7 +332,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
                 }
             }
         }
-        else d[k] = in ? inv_diag_cg(__ldg(a.diag + lo + i)) : 0.0;
+        else d[k] = in ? inv_diag_cg(a.A.diag(lo + i)) : 0.0;
         R.put(i, 0, x[k]);
     }
     tm.sync();
@@ -303,7 +342,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
     int it = 0, conv = 0;
     {
         double s[K][3];  // r.z, r.r, b.b
-        unsigned long long m[2] = {0, 0};
+        unsigned long long m[3] = {0, 0, 0};  // |r|, |b|, a row that does not fit
 #pragma unroll
         for (int k = 0; k < K; ++k)
         {
@@ -318,8 +357,9 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
             s[k][2] = bi * bi;
             m[0] = max(m[0], mag_bits(r[k]));
             m[1] = max(m[1], mag_bits(bi));
+            if (Mat::checked && i < cnt && a.A.end(lo + i) - a.A.first(lo + i) > kResW) m[2] = mag_bits(1.0);
         }
-        tm.reduce(s, m, [&](const double (&v)[5]) {
+        tm.reduce(s, m, [&](const double (&v)[6]) {
             init = (isnan(v[3]) || isnan(v[4])) ? NAN : (two ? sqrt(v[1]) : v[3]);
             bn = smax(two ? sqrt(v[2]) : (isnan(v[4]) ? 0.0 : v[4]), 1e-300);
             rz = v[0];
@@ -330,10 +370,16 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
                 fin = init;
                 go = false;
             }
+            if (Mat::checked && v[5] > 0.0)
+            {
+                it = -1;  // not this kernel's matrix: x is left as it was
+                go = false;
+            }
             if (threadIdx.x == 0)
             {
                 sc.go = go;
                 sc.beta = 0.0;
+                sc.fits = it >= 0;
             }
         });
     }
@@ -426,7 +472,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
     for (int k = 0; k < K; ++k)
     {
         const int i = threadIdx.x + k * kTeamThreads;
-        if (i < cnt) a.x[lo + i] = x[k];
+        if (i < cnt && sc.fits) a.x[lo + i] = x[k];
     }
     if (tm.rank == 0 && threadIdx.x == 0)
     {
@@ -446,11 +492,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg a, PersArgs 
     tm.finish();
 }
 
+template <class Mat>
 struct PersBi
 {
-    DMat A;
-    const double* val;
-    const double* diag;
+    Mat A;
     V3P b, x;
     V3P g;  // a grid team's copy of the gather vector
 };
@@ -467,17 +512,17 @@ struct BiScalars
 /// launch solves the component of its number: the components share only the
 /// matrix, so as teams of their own they take a third of the gathers and of
 /// the reduction each, and none waits for another that needs more iterations.
-template <int K, class Team, int NC>
-__global__ void __launch_bounds__(kTeamThreads, 1) k_pers_bicg(PersBi a, PersArgs t)
+template <int K, class Team, int NC, class Mat>
+__global__ void __launch_bounds__(kTeamThreads, 1) k_pers_bicg(PersBi<Mat> a, PersArgs t)
 {
     __shared__ TeamSmem smem;
     __shared__ BiScalars sc;
     extern __shared__ __align__(16) unsigned char dyn[];
     Team tm(smem, t.g);
     const int q0 = NC == 1 ? tm.team : 0;  // the team's first component
-    const int n = a.A.n, lo = min(n, tm.rank * t.chunk), cnt = min(n - lo, t.chunk);
+    const int n = a.A.n(), lo = min(n, tm.rank * t.chunk), cnt = min(n - lo, t.chunk);
     Resident<K, NC, Team, resident_regs(K, NC, false)> R(dyn, NC == 1 ? V3P{{a.g.c[q0], a.g.c[q0], a.g.c[q0]}} : a.g, lo, cnt);
-    R.load(a.A, a.val, t.chunk, tm.rank);
+    R.load(a.A, t.chunk, tm.rank);
     const int lane = threadIdx.x & 31, mine = lane < NC ? lane : 0;  // the component this lane advances (warp 0)
     unsigned long long none[1] = {0};
     constexpr bool kXs = resident_xs(K, NC);
@@ -492,7 +537,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_bicg(PersBi a, PersArg
     for (int k = 0; k < K; ++k)
     {
         const int i = threadIdx.x + k * kTeamThreads;
-        id[k] = i < cnt ? inv_diag_bicg(__ldg(a.diag + lo + i)) : 0.0;
+        id[k] = i < cnt ? inv_diag_bicg(a.A.diag(lo + i)) : 0.0;
 #pragma unroll
         for (int q = 0; q < NC; ++q)
         {
@@ -741,6 +786,57 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_bicg(PersBi a, PersArg
         }
     }
     tm.finish();
+}
+
+// ---- host side ----------------------------------------------------------------
+
+// rows per thread that registers and shared memory hold: one component, and
+// the three-component BiCGStab
+constexpr int kRes1K = kTeamRowsMax, kRes3K = 2;
+
+/// f(std::integral_constant<int, K>) for 1 <= K <= Kmax
+template <int Kmax, class F>
+void dispatchK(int K, F&& f)
+{
+    if constexpr (Kmax > 1)
+        if (K < Kmax) return dispatchK<Kmax - 1>(K, f);
+    f(std::integral_constant<int, Kmax>{});
+}
+
+inline TeamMem teamMem(const TeamPlan& tp, int n, unsigned* count, double* part, int* failed)
+{
+    return TeamMem{tp.blocks, count, part, (n + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, failed};
+}
+/// doubles of `part` for a system of n rows in one team, and in any plan
+constexpr size_t teamPartMax(int n) { return 2 * kTeamVals * (static_cast<size_t>(n) / kGroupRows + 1); }
+inline size_t teamPartSize(int n) { return kTeamsMax * 2 * kTeamVals * (static_cast<size_t>(n) / kGroupRows + 1); }
+
+/// A whole-solve kernel as `teams` teams of the plan on stream s.
+template <class Kern, class A>
+void launchTeam(const TeamPlan& tp, int teams, Kern kernel, const A& args, const PersArgs& t, size_t smem, cudaStream_t s)
+{
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(static_cast<unsigned>(tp.blocks * teams));
+    cfg.blockDim = dim3(kTeamThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    if (tp.cluster)
+    {
+        if (tp.blocks > 8) CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = static_cast<unsigned>(tp.blocks);
+        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    }
+    else
+    {
+        at[0].id = cudaLaunchAttributeCooperative;
+        at[0].val.cooperative = 1;
+    }
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    CFG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args, t));
 }
 
 }  // namespace cfg

@@ -635,8 +635,6 @@ Ctx::~Ctx()
     if (ownStream_) cudaStreamDestroy(stream_);
 }
 
-namespace
-{
 /// The largest cluster of whole-solve blocks the device runs: 16 (a
 /// non-portable size, which a partitioned GPU may not have), else 8, else 0.
 int largestCluster(int device)
@@ -646,7 +644,7 @@ int largestCluster(int device)
     std::lock_guard<std::mutex> lock(mu);
     const auto it = known.find(device);
     if (it != known.end()) return it->second;
-    const auto kernel = k_pers_cg<4, ClusterTeam, true>;
+    const auto kernel = k_pers_cg<4, ClusterTeam, true, SellView>;
     const size_t smem = resident_smem(4, 1, false);
     int best = 0;
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
@@ -670,7 +668,6 @@ int largestCluster(int device)
     known[device] = best;
     return best;
 }
-}  // namespace
 
 void Ctx::buildDevice()
 {
@@ -1045,7 +1042,7 @@ void Ctx::buildDevice()
     CFG_CUDA(cudaMallocHost(&stHost_, sizeof(SolveState)));
     CFG_CUDA(cudaMallocHost(&scalHost_, sizeof(double) * S_COUNT));
     teamCount_ = alloc<unsigned>(kTeamsMax * kCountStride);
-    teamPart_ = alloc<double>(kTeamsMax * 2 * kTeamVals * (static_cast<size_t>(nC) / kGroupRows + 1));
+    teamPart_ = alloc<double>(teamPartSize(nC));
     clusterMax_ = largestCluster(device_);
     {
         int coop = 0;
@@ -1465,13 +1462,6 @@ std::string ptrKey(const char* kind, std::initializer_list<const void*> ps, int 
 }
 }  // namespace
 
-namespace
-{
-// rows per thread that registers and shared memory hold: one component, and
-// the three-component BiCGStab
-constexpr int kRes1K = 4, kRes3K = 2;
-}  // namespace
-
 /// The team of a solve of nComp components, measured on jittered channels
 /// (Jacobi momentum and pressure, one outer iteration, B200; per-iteration
 /// kernels -> team): a cluster per component up to 16 blocks x 4 rows per
@@ -1484,32 +1474,25 @@ constexpr int kRes1K = 4, kRes3K = 2;
 /// per-iteration kernels.  Detail blocks and captured passes run side by
 /// side with others on the device and never take a grid, which wants every
 /// SM at once: their clusters do not depend on the schedule.
-Ctx::TeamPlan Ctx::teamPlan(int nComp, bool bicg) const
+TeamPlan teamPlanOf(int n, int nComp, int clusterMax, int sms, bool gridOk)
 {
     TeamPlan tp;
-    // per-kernel event timing needs the per-iteration kernels; longer rows
-    // do not fit the resident layout
-    if (ktime_ || maxW_ > kResW) return tp;
-    const int n = dm_.nC;
     // rows per block in whole groups of 256 (the unit of a sum's order)
     const int groups = (n + kGroupRows - 1) / kGroupRows;
+    if (groups > kGroupsMax) return tp;
     auto perBlock = [&](int blocks) { return (groups + blocks - 1) / blocks; };
-    // more groups than team_final_sum adds; a scalar equation's sums keep the
-    // per-iteration kernels' order, which has one row per thread up to G rows
-    if (groups > 768 || (bicg && nComp == 1 && n > initGS_ * TPB)) return tp;
     auto perThread = [&](int blocks) { return (perBlock(blocks) * kGroupRows + kTeamThreads - 1) / kTeamThreads; };
-    const bool gridOk = coopOk_ && !detail_ && !devLoop_;
-    if (clusterMax_ > 0 && perThread(clusterMax_) <= kRes1K)
+    if (clusterMax > 0 && perThread(clusterMax) <= kRes1K)
     {
         tp.cluster = true;
         tp.blocks = 1;
-        while (tp.blocks < clusterMax_ && perThread(tp.blocks) > 1) tp.blocks *= 2;
+        while (tp.blocks < clusterMax && perThread(tp.blocks) > 1) tp.blocks *= 2;
     }
-    else if (gridOk && perThread(sms_ / nComp) <= kRes1K)
-        tp.blocks = sms_ / nComp;
-    else if (gridOk && nComp == 3 && perThread(sms_) <= kRes3K)
+    else if (gridOk && perThread(sms / nComp) <= kRes1K)
+        tp.blocks = sms / nComp;
+    else if (gridOk && nComp == 3 && perThread(sms) <= kRes3K)
     {
-        tp.blocks = sms_;
+        tp.blocks = sms;
         tp.NC = 3;
     }
     if (tp.blocks)
@@ -1520,65 +1503,41 @@ Ctx::TeamPlan Ctx::teamPlan(int nComp, bool bicg) const
     return tp;
 }
 
+TeamPlan Ctx::teamPlan(int nComp, bool bicg) const
+{
+    // per-kernel event timing needs the per-iteration kernels; longer rows do
+    // not fit the resident layout; a scalar equation's sums keep the order of
+    // the per-iteration kernels, which have one row per thread up to initGS_
+    // blocks
+    if (ktime_ || maxW_ > kResW || (bicg && nComp == 1 && dm_.nC > initGS_ * TPB)) return TeamPlan{};
+    return teamPlanOf(dm_.nC, nComp, clusterMax_, sms_, coopOk_ && !detail_ && !devLoop_);
+}
+
 /// Launches a whole-solve kernel as its team.
 template <class Kern, class A>
 void Ctx::teamLaunch(const TeamPlan& tp, int teams, Kern kernel, const A& args, size_t smem, double tol, int maxIter,
                      int normType)
 {
-    const PersArgs t{tol, maxIter, normType, tp.chunk, st_, tally_, {tp.blocks, teamCount_, teamPart_,
-                     (dm_.nC + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, teamFailed_}};
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(static_cast<unsigned>(tp.blocks * teams));
-    cfg.blockDim = dim3(kTeamThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = stream_;
-    cudaLaunchAttribute at[1];
-    CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    if (tp.cluster)
-    {
-        if (tp.blocks > 8) CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = static_cast<unsigned>(tp.blocks);
-        at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
-    }
-    else
-    {
-        at[0].id = cudaLaunchAttributeCooperative;
-        at[0].val.cooperative = 1;
-    }
-    cfg.attrs = at;
-    cfg.numAttrs = 1;
-    CFG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args, t));
+    const PersArgs t{tol, maxIter, normType, tp.chunk, st_, tally_, teamMem(tp, dm_.nC, teamCount_, teamPart_, teamFailed_)};
+    launchTeam(tp, teams, kernel, args, t, smem, stream_);
     launchCheck("team_solve");
 }
-
-namespace
-{
-/// f(std::integral_constant<int, K>) for 1 <= K <= Kmax
-template <int Kmax, class F>
-void dispatchK(int K, F&& f)
-{
-    if constexpr (Kmax > 1)
-        if (K < Kmax) return dispatchK<Kmax - 1>(K, f);
-    f(std::integral_constant<int, Kmax>{});
-}
-}  // namespace
 
 void Ctx::teamBi(const TeamPlan& tp, int nComp, const double* vals, const double* diag, V3P b, V3P x, double tol,
                  int maxIter)
 {
-    const PersBi a{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag, b, x, bz_};
+    const PersBi<SellView> a{{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag}, b, x, bz_};
     if (tp.NC == 3)
         dispatchK<kRes3K>(tp.K, [&](auto Kc) {
             constexpr int K = decltype(Kc)::value;
-            teamLaunch(tp, 1, k_pers_bicg<K, GridTeam, 3>, a, resident_smem(K, 3, false), tol, maxIter, 0);
+            teamLaunch(tp, 1, k_pers_bicg<K, GridTeam, 3, SellView>, a, resident_smem(K, 3, false), tol, maxIter, 0);
         });
     else
         dispatchK<kRes1K>(tp.K, [&](auto Kc) {
             constexpr int K = decltype(Kc)::value;
             const size_t smem = resident_smem(K, 1, false);
-            if (tp.cluster) teamLaunch(tp, nComp, k_pers_bicg<K, ClusterTeam, 1>, a, smem, tol, maxIter, 0);
-            else teamLaunch(tp, nComp, k_pers_bicg<K, GridTeam, 1>, a, smem, tol, maxIter, 0);
+            if (tp.cluster) teamLaunch(tp, nComp, k_pers_bicg<K, ClusterTeam, 1, SellView>, a, smem, tol, maxIter, 0);
+            else teamLaunch(tp, nComp, k_pers_bicg<K, GridTeam, 1, SellView>, a, smem, tol, maxIter, 0);
         });
 }
 
@@ -1586,11 +1545,11 @@ template <bool kDic>
 void Ctx::teamCg(const TeamPlan& tp, const double* vals, const double* diag, const double* b, double* x,
                  const double* rDinv, double tol, int maxIter, int normType)
 {
-    const PersCg a{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag, b, x, cp_, rDinv, dColour_, dic_.nColours};
+    const PersCg<SellView> a{{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag}, b, x, cp_, rDinv, dColour_, dic_.nColours};
     dispatchK<kRes1K>(tp.K, [&](auto Kc) {
         constexpr int K = decltype(Kc)::value;
-        if (tp.cluster) teamLaunch(tp, 1, k_pers_cg<K, ClusterTeam, kDic>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
-        else teamLaunch(tp, 1, k_pers_cg<K, GridTeam, kDic>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
+        if (tp.cluster) teamLaunch(tp, 1, k_pers_cg<K, ClusterTeam, kDic, SellView>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
+        else teamLaunch(tp, 1, k_pers_cg<K, GridTeam, kDic, SellView>, a, resident_smem(K, 1, !kDic), tol, maxIter, normType);
     });
 }
 

@@ -6,6 +6,7 @@
 
 #include "ctx.h"
 #include "solvers.cuh"
+#include "persist.cuh"
 
 namespace cfg
 {
@@ -52,6 +53,99 @@ __global__ void k_diag_from_sell(DMat A, const int* __restrict__ isDiag, const d
     }
 }
 
+/// The solve as one resident kernel that reads the caller's CSR as it is:
+/// one allocation, the arrays copied in, the kernel, the solution copied out.
+/// False when the system does not fit (a row of more than kResW entries, more
+/// rows than a team holds).  A 30,044-row BiCGStab call took 9.4 ms with the
+/// SELL conversion on the host, an allocation per vector and four launches
+/// per iteration.
+bool residentSolve(int device, int n, int maxRow, const int64_t* rs, const int64_t* cols, const double* vals,
+                   const double* b, double* x, double tol, int maxIter, int method, cfg_solver_report* rep)
+{
+    int sms = 0, coop = 0;
+    CFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+    CFG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+    const TeamPlan tp = maxRow <= kResW ? teamPlanOf(n, 1, largestCluster(device), sms, coop != 0) : TeamPlan{};
+    if (!tp.blocks) return false;
+    const size_t N = static_cast<size_t>(n), nnz = static_cast<size_t>(rs[n]);
+    size_t bytes = 0;
+    auto place = [&](size_t size) {
+        const size_t at = bytes;
+        bytes += (size + 255) / 256 * 256;
+        return at;
+    };
+    // the zeroed part first: counters, the failure flag and the state
+    const size_t oCount = place(kTeamsMax * kCountStride * sizeof(unsigned)), oFail = place(sizeof(int)),
+                 oState = place(sizeof(SolveState)), zeroed = bytes;
+    const size_t oRs = place((N + 1) * sizeof(int64_t)), oCols = place(nnz * sizeof(int64_t)),
+                 oVals = place(nnz * sizeof(double)), oB = place(N * sizeof(double)), oX = place(N * sizeof(double)),
+                 oG = place(N * sizeof(double)), oPart = place(teamPartSize(n) * sizeof(double));
+    cudaStream_t s;
+    CFG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    struct Guard
+    {
+        cudaStream_t s;
+        unsigned char* p = nullptr;
+        ~Guard()
+        {
+            cudaStreamSynchronize(s);
+            cudaFree(p);
+            cudaStreamDestroy(s);
+        }
+    } g{s};
+    CFG_CUDA(cudaMalloc(&g.p, bytes));
+    unsigned char* d = g.p;
+    auto in = [&](size_t at, const void* src, size_t size) {
+        if (size) CFG_CUDA(cudaMemcpyAsync(d + at, src, size, cudaMemcpyHostToDevice, s));
+    };
+    CFG_CUDA(cudaMemsetAsync(d, 0, zeroed, s));
+    in(oRs, rs, (N + 1) * sizeof(int64_t));
+    in(oCols, cols, nnz * sizeof(int64_t));
+    in(oVals, vals, nnz * sizeof(double));
+    in(oB, b, N * sizeof(double));
+    in(oX, x, N * sizeof(double));
+    using View = CsrView<long long>;
+    static_assert(sizeof(long long) == sizeof(int64_t), "64-bit indices");
+    const View A{n, reinterpret_cast<const long long*>(d + oRs), reinterpret_cast<const long long*>(d + oCols),
+                 reinterpret_cast<const double*>(d + oVals)};
+    double* const db = reinterpret_cast<double*>(d + oB);
+    double* const dx = reinterpret_cast<double*>(d + oX);
+    double* const dg = reinterpret_cast<double*>(d + oG);
+    SolveState* const st = reinterpret_cast<SolveState*>(d + oState);
+    const PersArgs t{tol, maxIter, 0, tp.chunk, st, nullptr,
+                     teamMem(tp, n, reinterpret_cast<unsigned*>(d + oCount), reinterpret_cast<double*>(d + oPart),
+                             reinterpret_cast<int*>(d + oFail))};
+    dispatchK<kRes1K>(tp.K, [&](auto Kc) {
+        constexpr int K = decltype(Kc)::value;
+        if (method == CFG_SOLVE_CG)
+        {
+            const PersCg<View> a{A, db, dx, dg, nullptr, nullptr, 0};
+            const size_t smem = resident_smem(K, 1, true);
+            if (tp.cluster) launchTeam(tp, 1, k_pers_cg<K, ClusterTeam, false, View>, a, t, smem, s);
+            else launchTeam(tp, 1, k_pers_cg<K, GridTeam, false, View>, a, t, smem, s);
+        }
+        else
+        {
+            const PersBi<View> a{A, V3P{{db, db, db}}, V3P{{dx, dx, dx}}, V3P{{dg, dg, dg}}};
+            const size_t smem = resident_smem(K, 1, false);
+            if (tp.cluster) launchTeam(tp, 1, k_pers_bicg<K, ClusterTeam, 1, View>, a, t, smem, s);
+            else launchTeam(tp, 1, k_pers_bicg<K, GridTeam, 1, View>, a, t, smem, s);
+        }
+    });
+    SolveState h;
+    int failed = 0;
+    CFG_CUDA(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s));
+    CFG_CUDA(cudaMemcpyAsync(&failed, d + oFail, sizeof failed, cudaMemcpyDeviceToHost, s));
+    CFG_CUDA(cudaMemcpyAsync(x, dx, N * sizeof(double), cudaMemcpyDeviceToHost, s));
+    CFG_CUDA(cudaStreamSynchronize(s));
+    if (failed) fail(CFG_ECUDA, "sparse solve: a wait inside a kernel ran out");
+    rep->iterations = h.it[0];
+    rep->converged = h.conv[0];
+    rep->initial_residual = h.init[0];
+    rep->final_residual = (h.conv[0] && h.it[0] == 0) ? h.init[0] : h.fin[0];
+    return true;
+}
+
 }  // namespace
 
 void Ctx::sparseSolve(int device, int64_t n64, const int64_t* rs, const int64_t* cols, const double* vals,
@@ -59,13 +153,16 @@ void Ctx::sparseSolve(int device, int64_t n64, const int64_t* rs, const int64_t*
 {
     if (n64 <= 0 || n64 >= (1LL << 30)) fail(CFG_EINVAL, "sparse solve: matrix size out of range");
     const int n = static_cast<int>(n64);
+    int maxRow = 0;
     for (int r = 0; r < n; ++r)
     {
+        maxRow = std::max<int>(maxRow, static_cast<int>(std::min<int64_t>(rs[r + 1] - rs[r], 1 << 30)));
         if (rs[r + 1] < rs[r]) fail(CFG_EINVAL, "sparse solve: row offsets not ascending");
         for (int64_t k = rs[r]; k < rs[r + 1]; ++k)
             if (cols[k] < 0 || cols[k] >= n) fail(CFG_EINVAL, "sparse solve: column out of range");
     }
     CFG_CUDA(cudaSetDevice(device));
+    if (rs[0] == 0 && residentSolve(device, n, maxRow, rs, cols, vals, b, x, tol, maxIter, method, rep)) return;
     cudaStream_t s;
     CFG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
     struct StreamGuard

@@ -21,6 +21,7 @@
 
 #include "ctx.h"
 #include "solvers.cuh"
+#include "persist.cuh"
 
 namespace cfg
 {
@@ -32,7 +33,10 @@ constexpr int kStaticMaxBlocks = (kStaticMaxRows + RPT * TPB - 1) / (RPT * TPB);
 constexpr size_t kVecBytes = sizeof(double) * kStaticMaxRows;
 constexpr size_t kPartialBytes = sizeof(double) * 16 * kStaticMaxBlocks;
 constexpr size_t kStateBytes = (sizeof(SolveState) + 255) / 256 * 256;
-// layout: r, p, Ap, diag (one vector each), block partials, solver state
+// layout: r, p, Ap, diag (one vector each), block partials, solver state; the
+// resident kernel (persist.cuh) keeps a grid team's partials in r, its gather
+// vector in p and its counters and failure flag in Ap
+static_assert(teamPartMax(kStaticMaxRows) * sizeof(double) <= sizeof(double) * kStaticMaxRows, "partials fit a vector");
 constexpr size_t kScratchBytes = 4 * kVecBytes + kPartialBytes + kStateBytes;
 
 static __device__ __align__(256) unsigned char g_pcgScratch[kScratchBytes];
@@ -61,9 +65,11 @@ unsigned char* scratchOn(int device)
 /// Every field of the solver state cleared (tickets, flags, counters), then
 /// the tolerance and iteration limit set: the array keeps the previous
 /// call's contents.
-__global__ void k_static_state_init(SolveState* st, double tol, int maxIter)
+__global__ void k_static_state_init(SolveState* st, double tol, int maxIter, unsigned* count, int* failed)
 {
     if (blockIdx.x != 0 || threadIdx.x != 0) return;
+    for (int i = 0; i < kTeamsMax * kCountStride; ++i) count[i] = 0;
+    *failed = 0;
     unsigned char* b = reinterpret_cast<unsigned char*>(st);
     for (size_t i = 0; i < sizeof(SolveState); ++i) b[i] = 0;
     st->tol = tol;
@@ -225,8 +231,45 @@ extern "C" int cfg_pcg_solve_static(int32_t device, int64_t n64, const int32_t* 
         double* partials = reinterpret_cast<double*>(base + 4 * kVecBytes);
         SolveState* st = reinterpret_cast<SolveState*>(base + 4 * kVecBytes + kPartialBytes);
         cudaStream_t s = static_cast<cudaStream_t>(stream);
+        unsigned* count = reinterpret_cast<unsigned*>(Ap);
+        int* failed = reinterpret_cast<int*>(count + kTeamsMax * kCountStride);
+        // one resident kernel while the rows fit (persist.cuh checks their
+        // lengths and leaves x alone when one does not): on a 63^3 system 55 us
+        // an iteration as three launches over uncoalesced CSR rows
+        int sms = 0, coop = 0;
+        CFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
+        CFG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
+        if (const TeamPlan tp = teamPlanOf(n, 1, largestCluster(device), sms, coop != 0); tp.blocks)
+        {
+            k_static_state_init<<<1, 1, 0, s>>>(st, tol, maxIter, count, failed);
+            CFG_CUDA(cudaGetLastError());
+            using View = CsrView<int>;
+            const PersCg<View> a{View{n, rowStart, cols, vals}, b, x, p, nullptr, nullptr, 0};
+            const PersArgs t{tol, maxIter, 0, tp.chunk, st, nullptr, teamMem(tp, n, count, r, failed)};
+            dispatchK<kRes1K>(tp.K, [&](auto Kc) {
+                constexpr int K = decltype(Kc)::value;
+                const size_t smem = resident_smem(K, 1, true);
+                if (tp.cluster) launchTeam(tp, 1, k_pers_cg<K, ClusterTeam, false, View>, a, t, smem, s);
+                else launchTeam(tp, 1, k_pers_cg<K, GridTeam, false, View>, a, t, smem, s);
+            });
+            SolveState h;
+            int bad = 0;
+            CFG_CUDA(cudaMemcpyAsync(&h, st, sizeof(SolveState), cudaMemcpyDeviceToHost, s));
+            CFG_CUDA(cudaMemcpyAsync(&bad, failed, sizeof(int), cudaMemcpyDeviceToHost, s));
+            CFG_CUDA(cudaStreamSynchronize(s));
+            if (bad) fail(CFG_ECUDA, "cfg_pcg_solve_static: a wait inside a kernel ran out");
+            if (h.it[0] >= 0)
+            {
+                report->iterations = h.it[0];
+                report->converged = h.conv[0];
+                report->initial_residual = h.init[0];
+                report->final_residual = (h.conv[0] && h.it[0] == 0) ? h.init[0] : h.fin[0];
+                if (switched) cudaSetDevice(prev);
+                return CFG_OK;
+            }
+        }
         const int G = (n + RPT * TPB - 1) / (RPT * TPB);
-        k_static_state_init<<<1, 1, 0, s>>>(st, tol, maxIter);
+        k_static_state_init<<<1, 1, 0, s>>>(st, tol, maxIter, count, failed);
         k_static_cg_init<<<G, TPB, 0, s>>>(n, rowStart, cols, vals, b, x, r, p, d, partials, st);
         CFG_CUDA(cudaGetLastError());
         int allDone = 0;

@@ -35,6 +35,8 @@ constexpr int kClusterMax = 16;  // blocks of the largest cluster (non-portable 
 constexpr int kGroupRows = TPB;  // rows of one partial sum
 constexpr int kTeamRowsMax = 4;  // rows per thread (two partials each per block)
 constexpr int kPartMax = 2 * kTeamRowsMax;
+constexpr int kGridFold = 4;     // partials per thread of a grid team's final sum
+constexpr int kGroupsMax = 256 * kGridFold;  // most groups of a system
 
 /// Magnitude as an ordered integer: larger magnitudes compare larger and a
 /// NaN above every number, so one integer maximum carries both |v|inf and
@@ -167,7 +169,7 @@ __device__ __forceinline__ void team_block_reduce(TeamSmem& sm, int par, const d
 }
 
 /// final_sum over the partials, from the barrier that made them visible on:
-/// its thread t holds partials t, t + 256, t + 512; a tree over the lanes of
+/// its thread t holds partials t, t + 256, ...; a tree over the lanes of
 /// each of its eight warps here, one over the eight in warp 0, which calls f.
 /// sum(q, b) is partial b of sum q, top(q, b) block b's maximum q; all of a
 /// warp's loads are under way before the first is used.
@@ -350,7 +352,7 @@ struct GridTeam
         }
         __syncthreads();
         const double* part = part0 + static_cast<size_t>(par) * kTeamVals * groups;
-        team_final<3, NS, NM>(
+        team_final<kGridFold, NS, NM>(
             sm, groups, min(nb, groups), [&](int q, int b) { return __ldcg(part + q * groups + b); },
             [&](int q, int b) { return __ldcg(part + (NS + q) * groups + b); }, f);
         par ^= 1;
