@@ -1450,7 +1450,7 @@ int coarseKernels(const AmgState& a, const Smoother& sm)
 }
 }  // namespace
 
-void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single)
+void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single, bool swept)
 {
     if (!amg_) fail(CFG_EINVAL, "amg: the hierarchy is not set up (amgValues)");
     AmgState& a = *amg_;
@@ -1459,9 +1459,12 @@ void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bo
     const int* stop = st ? &st->done : nullptr;
     const int Wsel = maxW_ <= 7 ? 7 : (maxW_ <= 16 ? 16 : 0);
     const AmgLevel& V = a.lv[0];
-    const auto pre0 = Wsel == 7 ? k_amg_pre0<7> : (Wsel == 16 ? k_amg_pre0<16> : k_amg_pre0<0>);
-    launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32, V.dinv,
-            r, V.x, V.r);
+    if (!swept)
+    {
+        const auto pre0 = Wsel == 7 ? k_amg_pre0<7> : (Wsel == 16 ? k_amg_pre0<16> : k_amg_pre0<0>);
+        launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
+                V.dinv, r, V.x, V.r);
+    }
     const Smoother sm = single ? singleSweeps() : smootherOf(a);
     coarseCycle<float>(a, pdl_, sms_, stream_, stop, kScale, sm);
     // one block partial per block: the grid is at most G_ blocks, which
@@ -1599,22 +1602,29 @@ __global__ void __launch_bounds__(TPB) k_fcgd_init(DMat A, const double* __restr
     }
 }
 
-/// q = A p with p.r and p.q; alpha = p.r / p.q, or done on a breakdown
-template <int W>
-__global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restrict__ val, const double* __restrict__ p,
+/// q = A p with p.r and p.q; alpha = p.r / p.q, or done on a breakdown.
+/// kForm: p = z + beta p is formed here, per column as the row is read (the
+/// old p stays for the other rows, the new one goes to pNew); beta is 0 in
+/// the first iteration and p zero.
+template <int W, bool kForm>
+__global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restrict__ val, const double* __restrict__ z,
+                                                   const double* __restrict__ p, double* __restrict__ pNew,
                                                    const double* __restrict__ r, double* __restrict__ q,
                                                    double* partials, FcgState* st)
 {
     pdl_entry();
     if (st->done) return;
+    const double be = st->beta;
     double s[2] = {0.0, 0.0};
-    const double* xs[1] = {p};
     FOR_ROWS(c, A.n)
     {
         double y[1];
-        spmv_row<W, 1>(A, val, c, xs, y);
+        spmv_row_gather<W, 1>(A, val, c, y, [&](int col, double (&xv)[1]) {
+            xv[0] = kForm ? __ldg(z + col) + be * __ldg(p + col) : __ldg(p + col);
+        });
         q[c] = y[0];
-        const double pc = p[c];
+        const double pc = kForm ? z[c] + be * p[c] : p[c];
+        if (kForm) pNew[c] = pc;
         s[0] += pc * r[c];
         s[1] += pc * y[0];
     }
@@ -1640,23 +1650,9 @@ __global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restr
     }
 }
 
-/// x += alpha p, r -= alpha q, |r|2 and the stopping test
-__global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* __restrict__ p, const double* __restrict__ q,
-                                                     double* __restrict__ x, double* __restrict__ r, double* partials,
-                                                     FcgState* st)
+/// The end of an update: |r| from the block values in s, and the stopping test
+__device__ __forceinline__ void fcg_update_end(double (&s)[1], bool inf, double* partials, FcgState* st)
 {
-    pdl_entry();
-    if (st->done) return;
-    const bool inf = st->normType == 0;
-    const double al = st->alpha;
-    double s[1] = {0.0};
-    FOR_ROWS(c, n)
-    {
-        x[c] = x[c] + al * p[c];
-        const double rc = r[c] - al * q[c];
-        r[c] = rc;
-        s[0] = inf ? smax(s[0], fabs(rc)) : s[0] + rc * rc;
-    }
     if (inf) block_max<1>(s);
     else block_sum<1>(s);
     if (threadIdx.x == 0) partials[blockIdx.x] = s[0];
@@ -1681,15 +1677,75 @@ __global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* __rest
     }
 }
 
-/// p = z + beta p (beta = 0 gives p = z)
-__global__ void __launch_bounds__(TPB) k_fcgd_p(int n, const double* __restrict__ z, double* __restrict__ p,
-                                                const FcgState* st, int first)
+/// x += alpha p, r -= alpha q, |r| and the stopping test
+__global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* __restrict__ p, const double* __restrict__ q,
+                                                     double* __restrict__ x, double* __restrict__ r, double* partials,
+                                                     FcgState* st)
 {
     pdl_entry();
     if (st->done) return;
-    const double be = first ? 0.0 : st->beta;
-    FOR_ROWS(c, n) p[c] = first ? z[c] : z[c] + be * p[c];
+    const bool inf = st->normType == 0;
+    const double al = st->alpha;
+    double s[1] = {0.0};
+    FOR_ROWS(c, n)
+    {
+        x[c] = x[c] + al * p[c];
+        const double rc = r[c] - al * q[c];
+        r[c] = rc;
+        s[0] = inf ? smax(s[0], fabs(rc)) : s[0] + rc * rc;
+    }
+    fcg_update_end(s, inf, partials, st);
 }
+
+/// p = z + beta p
+__global__ void __launch_bounds__(TPB) k_fcgd_p(int n, const double* __restrict__ z, double* __restrict__ p,
+                                                const FcgState* st)
+{
+    pdl_entry();
+    if (st->done) return;
+    const double be = st->beta;
+    FOR_ROWS(c, n) p[c] = z[c] + be * p[c];
+}
+
+/// x += alpha p, r -= alpha q with |r| and the stopping test, and the
+/// V-cycle's finest first sweep and residual of the new r (k_amg_pre0), which
+/// is formed per column as the row is read (the old r stays for the other
+/// rows).  When the test is met the sweep has been for nothing, once a solve.
+template <int W>
+__global__ void __launch_bounds__(TPB) k_fcgd_update_pre0(DMat A, const float* __restrict__ val,
+                                                          const float* __restrict__ dinv, const double* __restrict__ p,
+                                                          const double* __restrict__ q, double* __restrict__ x,
+                                                          const double* __restrict__ r, double* __restrict__ rNew,
+                                                          float* __restrict__ xs, float* __restrict__ rs,
+                                                          double* partials, FcgState* st)
+{
+    pdl_entry();
+    if (st->done) return;
+    const bool inf = st->normType == 0;
+    const double al = st->alpha;
+    double s[1] = {0.0};
+    FOR_ROWS(c, A.n)
+    {
+        const double rc = r[c] - al * q[c];
+        const float sum = sell_row<W>(A, val, c, [&](int j) {
+            return kOmega * __ldg(dinv + j) * static_cast<float>(__ldg(r + j) - al * __ldg(q + j));
+        });
+        const float bc = static_cast<float>(rc);
+        x[c] = x[c] + al * p[c];
+        rNew[c] = rc;
+        xs[c] = kOmega * dinv[c] * bc;
+        rs[c] = bc - sum;
+        s[0] = inf ? smax(s[0], fabs(rc)) : s[0] + rc * rc;
+    }
+    fcg_update_end(s, inf, partials, st);
+}
+
+/// Up to this many rows the search direction is formed in the product and the
+/// update in the first sweep: two launches fewer per iteration for a second
+/// gathered vector in each (158k-cell PISO step 9.5 -> 8.4 ms, 55k-tet Poisson
+/// 3.27 -> 3.16 ms; above it the gathers cost more than the launches: 262k
+/// cells 31.4 -> 31.6 ms, 1.2M 16.4 -> 16.8 ms, 2M 158.7 -> 162.6 ms).
+constexpr int kFormRows = 200000;
 
 }  // namespace
 
@@ -1705,9 +1761,12 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     AmgState& a = *amg_;
     const int n = dm_.nC;
     const DMat A{n, dm_.mStart, dm_.mCol};
-    double* r = cr_;
+    // with `form`, r and p alternate between two vectors each: the kernels
+    // that form them read the old values at their neighbours
+    const bool form = n <= kFormRows;
+    double* const rr[2] = {cr_, br_.c[0]};
+    double* const pp[2] = {cp_, br_.c[1]};
     double* z = cz_;
-    double* p = cp_;
     double* q = cAp_;
     if (!a.st)
     {
@@ -1721,24 +1780,33 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     CFG_CUDA(cudaMemcpyAsync(a.st, &init, sizeof(FcgState), cudaMemcpyHostToDevice, stream_));
     auto spmvInit = [&](auto Wc) {
         constexpr int W = decltype(Wc)::value;
-        k_fcgd_init<W><<<GS_, TPB, 0, stream_>>>(A, vals, b, x, r, partials_, a.st);
+        k_fcgd_init<W><<<GS_, TPB, 0, stream_>>>(A, vals, b, x, rr[0], partials_, a.st);
     };
     const int Wsel = maxW_ <= 7 ? 7 : (maxW_ <= 16 ? 16 : 0);
     if (Wsel == 7) spmvInit(std::integral_constant<int, 7>{});
     else if (Wsel == 16) spmvInit(std::integral_constant<int, 16>{});
     else spmvInit(std::integral_constant<int, 0>{});
     launchCheck("fcgd_init");
-    amgCycle(r, z, nullptr, a.st, false);
-    launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, p, a.st, 1);
-    launchCheck("fcgd_p0");
-    const auto spmv = Wsel == 7 ? k_fcgd_spmv<7> : (Wsel == 16 ? k_fcgd_spmv<16> : k_fcgd_spmv<0>);
+    amgCycle(rr[0], z, nullptr, a.st, false);
+    CFG_CUDA(cudaMemsetAsync(pp[0], 0, static_cast<size_t>(n) * sizeof(double), stream_));
+    const auto pick = [&](auto a7, auto a16, auto a0) { return Wsel == 7 ? a7 : (Wsel == 16 ? a16 : a0); };
+    const auto spmv = form ? pick(k_fcgd_spmv<7, true>, k_fcgd_spmv<16, true>, k_fcgd_spmv<0, true>)
+                           : pick(k_fcgd_spmv<7, false>, k_fcgd_spmv<16, false>, k_fcgd_spmv<0, false>);
+    const auto update = pick(k_fcgd_update_pre0<7>, k_fcgd_update_pre0<16>, k_fcgd_update_pre0<0>);
     const int spmvGrid = waveGrid(reinterpret_cast<const void*>(spmv), sms_, n);
-    auto iteration = [&]() {
-        launchK(pdl_, spmv, spmvGrid, TPB, 0, stream_, A, vals, p, r, q, partials_, a.st);
-        launchK(pdl_, k_fcgd_update, GS_, TPB, 0, stream_, n, p, q, x, r, partials_, a.st);
-        amgCycle(r, z, q, a.st, false);
-        launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, p, a.st, 0);
-        launchCheck("fcgd_iter", 3);
+    const int updateGrid = waveGrid(reinterpret_cast<const void*>(update), sms_, n);
+    // iteration k of a chunk; every chunk but a solve's last has an even
+    // number of them, so each begins with the vectors of index 0
+    auto iteration = [&](int k) {
+        const int o = form ? k & 1 : 0, w = form ? o ^ 1 : 0;
+        if (!form) launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, pp[0], a.st);
+        launchK(pdl_, spmv, spmvGrid, TPB, 0, stream_, A, vals, z, pp[o], pp[w], rr[o], q, partials_, a.st);
+        if (form)
+            launchK(pdl_, update, updateGrid, TPB, 0, stream_, A, a.vals32, a.lv[0].dinv, pp[w], q, x, rr[o], rr[w],
+                    a.lv[0].x, a.lv[0].r, partials_, a.st);
+        else launchK(pdl_, k_fcgd_update, GS_, TPB, 0, stream_, n, pp[0], q, x, rr[0], partials_, a.st);
+        amgCycle(rr[w], z, q, a.st, false, form);
+        launchCheck("fcgd_iter", form ? 1 : 3);
     };
     for (int launched = 0, chunk = 8;;)
     {
@@ -1756,7 +1824,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
         {
             cudaGraph_t g = nullptr;
             CFG_CUDA(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
-            for (int k = 0; k < m; ++k) iteration();
+            for (int k = 0; k < m; ++k) iteration(k);
             CFG_CUDA(cudaStreamEndCapture(stream_, &g));
             const cudaError_t e = cudaGraphInstantiate(&ge, g, 0);
             cudaGraphDestroy(g);
@@ -1765,8 +1833,8 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
         }
         if (ge) CFG_CUDA(cudaGraphLaunch(ge, stream_));
         else
-            for (int k = 0; k < m; ++k) iteration();
-        launches_ = counted + static_cast<int64_t>(m) * (3 + amgCycleKernels(kAmgPressure, false));
+            for (int k = 0; k < m; ++k) iteration(k);
+        launches_ = counted + static_cast<int64_t>(m) * ((form ? 1 : 3) + amgCycleKernels(kAmgPressure, false));
         launched += m;
         chunk = std::min(chunk * 2, 32);
     }

@@ -298,8 +298,10 @@ private:
     void amgValues(AmgUse use, const double* vals, const double* diag, const float* vals32);
     void amgApply(const double* r, double* z);
     /// single: one sweep before and after each correction on every level, else
-    /// the hierarchy's own smoothers on the coarse ones
-    void amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single);
+    /// the hierarchy's own smoothers on the coarse ones; swept: the finest
+    /// first sweep and residual are there already
+    void amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single,
+                  bool swept = false);
     /// mark(0) after the finest pre-sweep, mark(1) before the finest
     /// post-sweep (kernel timing), when given
     void amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, bool single,

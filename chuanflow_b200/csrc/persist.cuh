@@ -241,22 +241,21 @@ struct PersCg
 
 /// z = M^-1 r of the multicolour DIC (k_dic_fwd, k_dic_bwd) and this
 /// thread's r z: one team barrier between colours, z passed to the
-/// neighbours through the gather vector.
+/// neighbours through the gather vector.  On entry z = rDinv r is there
+/// already (the first colour has no lower entries), put before the last
+/// reduction, whose barrier made it visible.
 template <int K, class Team, class Res>
 __device__ __forceinline__ void pers_dic(Team& tm, Res& R, int C, const double (&r)[K], const double (&rd)[K],
                                            const int (&col)[K], const unsigned (&lower)[K], const unsigned (&upper)[K],
                                          double (&z)[K], double (&rz)[K][1])
 {
-#pragma unroll
-    for (int k = 0; k < K; ++k)
-    {
-        z[k] = rd[k] * r[k];  // the first colour has no lower entries
-        R.put(threadIdx.x + k * kTeamThreads, 0, z[k]);
-    }
     for (int c = 1; c < C; ++c)
     {
-        tm.sync();
-        if (tm.dead()) return;
+        if (c > 1)
+        {
+            tm.sync();
+            if (tm.dead()) return;
+        }
 #pragma unroll
         for (int k = 0; k < K; ++k)
         {
@@ -388,6 +387,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
     {
         if (go)
         {
+            // the gather vector held x until here
+#pragma unroll
+            for (int k = 0; k < K; ++k) R.put(threadIdx.x + k * kTeamThreads, 0, z[k]);
+            tm.sync();
             double s[K][1] = {};
             pers_dic<K>(tm, R, a.nColours, r, d, col, lower, upper, z, s);
             tm.reduce(s, none, [&](const double (&v)[2]) { rz = v[0]; });
@@ -432,7 +435,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
         {
             x[k] = x[k] + alpha * p[k];
             r[k] = r[k] - alpha * q[k];
-            if constexpr (!kDic) z[k] = d[k] * r[k];
+            z[k] = d[k] * r[k];
+            if constexpr (kDic) R.put(threadIdx.x + k * kTeamThreads, 0, z[k]);
             s2[k][0] = kDic ? 0.0 : r[k] * z[k];
             s2[k][1] = r[k] * r[k];
             m[0] = max(m[0], mag_bits(r[k]));
