@@ -1599,7 +1599,7 @@ void Ctx::runCG(const double* vals, const double* diag, const double* b, double*
         dispatchW(maxW_, [&](auto Wc) {
             constexpr int W = decltype(Wc)::value;
             k_cg_init<W><<<GS_, TPB, 0, stream_>>>(A, vals, diag, b, x, cr_, cp_, partials_, st_);
-            constexpr int CH = 8;
+            constexpr int CH = 24;  // iterations per test of the loop condition
             captureWhile((maxIter + CH - 1) / CH + 1, [&] {
                 for (int k = 0; k < CH; ++k)
                 {
@@ -1679,7 +1679,7 @@ void Ctx::runBiCG3(const double* vals, const double* diag, V3P b, V3P x, int nCo
             constexpr int W = decltype(Wc)::value;
             constexpr int NC = decltype(NCc)::value;
             k_bi_init<W, NC><<<GS_, TPB, 0, stream_>>>(A, vals, diag, bInvD_, b, x, br_, br0_, bp_, bv_, partials_, st_);
-            constexpr int CH = 4;
+            constexpr int CH = 16;  // iterations per test of the loop condition
             captureWhile((maxIter + CH - 1) / CH + 1, [&] {
                 for (int k = 0; k < CH; ++k)
                 {
@@ -1808,21 +1808,21 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
                 const std::function<void(int)> markZ = [&](int j) { tmark(k, 2 + j); };
                 const std::function<void(int)> markS = [&](int j) { tmark(k, 7 + j); };
                 tmark(k, 0);
-                launchK(pdl_, k_bia_p<3>, GS_, TPB, 0, stream_, n, br_, bp_, bv_, st_);
+                launchK(amgPdl(), k_bia_p<3>, GS_, TPB, 0, stream_, n, br_, bp_, bv_, st_);
                 tmark(k, 1);
                 amgCycle3(kAmgMomentum, cv(bp_), bz_, done, kAmgScaleMomentum, false,
                           ktime_ ? markZ : std::function<void(int)>{});
                 tmark(k, 4);
-                launchK(pdl_, k_bi_spmv1<W, 3>, GS_, TPB, 0, stream_, A, vals, bz_, bv_, br0_, partials_, st_);
+                launchK(amgPdl(), k_bi_spmv1<W, 3>, GS_, TPB, 0, stream_, A, vals, bz_, bv_, br0_, partials_, st_);
                 tmark(k, 5);
-                launchK(pdl_, k_bia_s<3>, GS_, TPB, 0, stream_, n, br_, bv_, bs_, st_);
+                launchK(amgPdl(), k_bia_s<3>, GS_, TPB, 0, stream_, n, br_, bv_, bs_, st_);
                 tmark(k, 6);
                 amgCycle3(kAmgMomentum, cv(bs_), bsh_, done, kAmgScaleMomentum, false,
                           ktime_ ? markS : std::function<void(int)>{});
                 tmark(k, 9);
-                launchK(pdl_, k_bia_spmv2<W, 3>, GS_, TPB, 0, stream_, A, vals, bsh_, bs_, bt_, partials_, st_);
+                launchK(amgPdl(), k_bia_spmv2<W, 3>, GS_, TPB, 0, stream_, A, vals, bsh_, bs_, bt_, partials_, st_);
                 tmark(k, 10);
-                launchK(pdl_, k_bia_x<3>, GS_, TPB, 0, stream_, n, x, bz_, bs_, bsh_, bt_, br_, br0_, partials_, st_);
+                launchK(amgPdl(), k_bia_x<3>, GS_, TPB, 0, stream_, n, x, bz_, bs_, bsh_, bt_, br_, br0_, partials_, st_);
                 tmark(k, 11);
                 launchCheck("bicga_iter", 0);
             });
@@ -1920,7 +1920,7 @@ void Ctx::dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T*
             k_cg_init<W, T><<<GS_, TPB, 0, stream_>>>(A, vals, diag, b, x, r, p, partials_, st_);
             dicApplyT<T>(D, r, z);
             k_cg_pz<T><<<GS_, TPB, 0, stream_>>>(dm_.nC, z, p, st_);
-            constexpr int CH = 8;
+            constexpr int CH = 24;  // iterations per test of the loop condition
             captureWhile((maxIter + CH - 1) / CH + 1, [&] {
                 for (int k = 0; k < CH; ++k)
                 {
