@@ -1462,15 +1462,15 @@ void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bo
     if (!swept)
     {
         const auto pre0 = Wsel == 7 ? k_amg_pre0<7> : (Wsel == 16 ? k_amg_pre0<16> : k_amg_pre0<0>);
-        launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
+        launchK(amgPdl(), pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
                 V.dinv, r, V.x, V.r);
     }
     const Smoother sm = single ? singleSweeps() : smootherOf(a);
-    coarseCycle<float>(a, pdl_, sms_, stream_, stop, kScale, sm);
+    coarseCycle<float>(a, amgPdl(), sms_, stream_, stop, kScale, sm);
     // one block partial per block: the grid is at most G_ blocks, which
     // partials_ holds
     const auto post0 = Wsel == 7 ? k_amg_post0<7> : (Wsel == 16 ? k_amg_post0<16> : k_amg_post0<0>);
-    launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
+    launchK(amgPdl(), post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
             V.dinv, r, V.r, z, q, partials_, st);
     launchCheck("amg_vcycle", amgCycleKernels(kAmgPressure, single));
 }
@@ -1490,13 +1490,13 @@ void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, boo
     float4* const x = reinterpret_cast<float4*>(V.x3);
     float4* const r = reinterpret_cast<float4*>(V.r3);
     const auto pre0 = Wsel == 7 ? k_amgv_pre0<7> : (Wsel == 16 ? k_amgv_pre0<16> : k_amgv_pre0<0>);
-    launchK(pdl_, pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32, V.dinv,
+    launchK(amgPdl(), pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32, V.dinv,
             b, x, r);
     if (mark) mark(0);
-    coarseCycle<float4>(a, pdl_, sms_, stream_, done, scale, single ? singleSweeps() : smootherOf(a));
+    coarseCycle<float4>(a, amgPdl(), sms_, stream_, done, scale, single ? singleSweeps() : smootherOf(a));
     if (mark) mark(1);
     const auto post0 = Wsel == 7 ? k_amgv_post0<7> : (Wsel == 16 ? k_amgv_post0<16> : k_amgv_post0<0>);
-    launchK(pdl_, post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32,
+    launchK(amgPdl(), post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32,
             V.dinv, b, r, z);
     launchCheck("amg_vcycle3", amgCycleKernels(use, single));
 }
@@ -1799,12 +1799,12 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     // number of them, so each begins with the vectors of index 0
     auto iteration = [&](int k) {
         const int o = form ? k & 1 : 0, w = form ? o ^ 1 : 0;
-        if (!form) launchK(pdl_, k_fcgd_p, GS_, TPB, 0, stream_, n, z, pp[0], a.st);
-        launchK(pdl_, spmv, spmvGrid, TPB, 0, stream_, A, vals, z, pp[o], pp[w], rr[o], q, partials_, a.st);
+        if (!form) launchK(amgPdl(), k_fcgd_p, GS_, TPB, 0, stream_, n, z, pp[0], a.st);
+        launchK(amgPdl(), spmv, spmvGrid, TPB, 0, stream_, A, vals, z, pp[o], pp[w], rr[o], q, partials_, a.st);
         if (form)
-            launchK(pdl_, update, updateGrid, TPB, 0, stream_, A, a.vals32, a.lv[0].dinv, pp[w], q, x, rr[o], rr[w],
+            launchK(amgPdl(), update, updateGrid, TPB, 0, stream_, A, a.vals32, a.lv[0].dinv, pp[w], q, x, rr[o], rr[w],
                     a.lv[0].x, a.lv[0].r, partials_, a.st);
-        else launchK(pdl_, k_fcgd_update, GS_, TPB, 0, stream_, n, pp[0], q, x, rr[0], partials_, a.st);
+        else launchK(amgPdl(), k_fcgd_update, GS_, TPB, 0, stream_, n, pp[0], q, x, rr[0], partials_, a.st);
         amgCycle(rr[w], z, q, a.st, false, form);
         launchCheck("fcgd_iter", form ? 1 : 3);
     };

@@ -427,12 +427,16 @@ private:
     int64_t launches_ = 0;
     bool ktime_ = false;
     bool useGraphs_ = true;
-    // CHUANFLOW_PDL=1: the host-driven solver loops (AMG V-cycles, the AMG
-    // flexible CG, the AMG-preconditioned BiCGStab) launch their kernels as
-    // programmatic dependents of the kernel before.  Off by default: on the
-    // 2M-cell channel it shortened the eagerly launched V-cycle's coarse part
-    // (108.6 -> 94.7 us) but lengthened the graph-replayed outer iteration
-    // (265.5 -> 269.9 ms), with the same results
+    // Programmatic dependent launch of the host-driven solver loops (AMG
+    // V-cycles, the AMG flexible CG, the AMG-preconditioned BiCGStab): each
+    // kernel's blocks are scheduled while the one before drains.  On up to
+    // kPdlRows rows, whose kernels last a few microseconds (55k-tet Poisson
+    // 3.02 -> 2.88 ms, 158k-cell PISO step 8.33 -> 7.96 ms); above, the
+    // waiting blocks hold the running kernel's slots (262k cells 42.6 -> 43.3
+    // ms, 2M 298 -> 302 ms before the sweeps' change).  CHUANFLOW_PDL=1: on
+    // every size.  The results are the same.
+    static constexpr int kPdlRows = 200000;
+    bool amgPdl() const { return pdl_ || dm_.nC <= kPdlRows; }
     bool pdl_ = false;
     std::map<std::string, cudaGraphExec_t> graphs_;
     static constexpr int kEvPerIter = 12;  // events per solver iteration of a chunk (timed segments + 1)
