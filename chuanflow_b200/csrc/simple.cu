@@ -1465,12 +1465,12 @@ std::string ptrKey(const char* kind, std::initializer_list<const void*> ps, int 
 /// The team of a solve of nComp components, measured on jittered channels
 /// (Jacobi momentum and pressure, one outer iteration, B200; per-iteration
 /// kernels -> team): a cluster per component up to 16 blocks x 4 rows per
-/// thread = 32,768 rows (1,320 rows 31 -> 6.9 ms, 16,000 rows 138 -> 35 ms,
-/// 22,743 rows 45 -> 14 ms; a grid there took 20, 71 and 21 ms, its barriers
-/// costing six of a cluster's); then a grid per component while the rows fit
-/// (62,720 rows 73 -> 36 ms, 102,400 rows 93 -> 45 ms for the pair of
-/// solvers), then one grid for the three together (131,544 rows, DIC: 58 ->
-/// 33 ms).  Larger systems stream from memory anyway and keep the
+/// thread = 32,768 rows (1,320 rows 31 -> 7.9 ms, 16,000 rows 146 -> 39 ms,
+/// 22,743 rows with k-epsilon 43 -> 17 ms; a grid there took 20, 71 and 21
+/// ms, its barriers costing six of a cluster's); then a grid per component
+/// while the rows fit (62,720 rows 70 -> 37 ms, 102,400 rows 93 -> 52 ms),
+/// then one grid for the three together (131,072 rows 100 -> 53 ms, with DIC
+/// 89 -> 54 ms).  Larger systems stream from memory anyway and keep the
 /// per-iteration kernels.  Detail blocks and captured passes run side by
 /// side with others on the device and never take a grid, which wants every
 /// SM at once: their clusters do not depend on the schedule.

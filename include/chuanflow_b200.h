@@ -404,11 +404,13 @@ int cfg_poisson_solve(cfg_ctx* ctx, const double* b, double* x, int32_t method, 
  * (plain aggregation, Galerkin gather lists; once per mesh), out[10] value
  * set-up ms (device Galerkin sums and the coarsest dense inverse). */
 int cfg_poisson_amg_setup(cfg_ctx* ctx, double out[11]);
-/* One V-cycle of that hierarchy, z = V(r) (host vectors, original order):
- * the preconditioner as CFG_POISSON_FCG_AMG applies it, for tests. */
+/* One V-cycle of that hierarchy with one damped-Jacobi sweep on either side
+ * of each coarse correction, z = V(r) (host vectors, original order), for
+ * tests.  CFG_POISSON_FCG_AMG applies the same cycle with two to four
+ * weighted sweeps on the coarse levels. */
 int cfg_poisson_amg_apply(cfg_ctx* ctx, const double* r, double* z);
-/* The three-component V-cycle the AMG momentum BiCGStab applies, on the
- * same hierarchy: r and z hold three vectors one after another (3 n
+/* The three-component form of that V-cycle (the AMG momentum BiCGStab's, with
+ * single sweeps), on the same hierarchy: r and z hold three vectors one after another (3 n
  * values); component q is skipped, its z left as given, when done[q] != 0.
  * Each applied component equals cfg_poisson_amg_apply of it, for tests. */
 int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32_t done[3]);
