@@ -116,6 +116,7 @@ struct AmgState
     // its entries (0: it does not fit, its kernels and k_amg_dense run)
     size_t tailSmem = 0;
     int tailNnz = 0;
+    bool tailCluster = false;  // k_amg_tail, else k_amg_tail_block
     int skewClass = 0;    // how far from symmetric the finest operator is (skewOf)
     double* skew = nullptr;
 };
@@ -725,11 +726,22 @@ __global__ void __launch_bounds__(TPB) k_amg_smooth_sell(const int* __restrict__
 
 constexpr int kTailMax = 1024;  // rows of the fused last aggregation level
 constexpr int kTailThreads = 1024;
-constexpr int kTailLanes = 4;
+// A cluster per vector above two entries per thread, one block below, where
+// a product is a few hundred cycles and the barriers between them would be
+// more.  Whole solves, block -> cluster: 55k tets (529 rows, 6,935 entries)
+// 2.87 -> 2.64 ms, 1.2M hexahedra (279, 4,725) 16.4 -> 15.8 ms, 2M-cell
+// channel (514, 9,450) 158.7 -> 155.4 ms, 262k-cell channel (458, 4,720 and
+// 269, 2,417) 29.0 -> 28.9 ms; 158k-cell PISO (135, 1,009) 7.97 -> 8.18 ms.
+constexpr int kTailClusterEntries = 2048;
+constexpr int kTailBlocks = 8;  // a cluster per vector
+constexpr int kTailLanes = 8;   // lanes of a row; lane l hands the row's value to block l
+static_assert(kTailLanes == kTailBlocks, "a lane per block");
+constexpr int kTailRows = kTailThreads / kTailLanes;
+static_assert(kTailMax <= kTailBlocks * kTailRows && kDenseMax <= kTailRows, "one row per group of lanes");
 
 struct TailLevel
 {
-    int n, nc, nnz;
+    int n, nc, nnz;  // nnz: most entries in one block's rows
     const int *rs, *cols, *agg, *ms, *mem;
     const float *val, *dinv, *dense;
     const float* b;  // this level's right-hand side and output: a vector's
@@ -739,25 +751,169 @@ struct TailLevel
     Sweeps w;
 };
 
-/// Shared-memory layout of k_amg_tail (4-byte words): the level's CSR
+/// block `rank`'s share of n rows begins at
+__host__ __device__ constexpr int tailFirst(int n, int rank) { return n * rank / kTailBlocks; }
+/// the most rows of one share
+__host__ __device__ constexpr int tailShare(int n) { return (n + kTailBlocks - 1) / kTailBlocks; }
+
+/// Shared-memory layout of a k_amg_tail block (4-byte words).  Its share of
+/// the level's CSR (rs, cols, val) and of the dense inverse's rows; whole:
+/// dinv, agg and the aggregates' member lists (ms nc + 1, mem n), the vectors
+/// b, x, r (n each), bc and xc (nc each).
+__host__ __device__ constexpr size_t tailSmemWords(int n, int nnz, int nc)
+{
+    return static_cast<size_t>(tailShare(n) + 1) + 2 * static_cast<size_t>(nnz) +
+           static_cast<size_t>(tailShare(nc)) * static_cast<size_t>(nc) + 6 * static_cast<size_t>(n) +
+           static_cast<size_t>(nc + 1) + 2 * static_cast<size_t>(nc);
+}
+
+/// An asynchronous copy of one word to shared address `to`.
+__device__ __forceinline__ void copyWord(unsigned to, const void* from)
+{
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(to), "l"(from) : "memory");
+}
+/// v at p of block `block` of the cluster
+__device__ __forceinline__ void putAt(float* p, int block, float v)
+{
+    unsigned at;
+    asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(static_cast<unsigned>(__cvta_generic_to_shared(p))), "r"(block));
+    asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(at), "f"(v) : "memory");
+}
+__device__ __forceinline__ void clusterArrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
+__device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+/// The last aggregation level (at most kTailMax rows) and the coarsest solve
+/// as one cluster per vector: the sweeps and the residual, restriction, dense
+/// solve, prolongation and the sweeps again.  Every block holds the vectors
+/// whole and an eighth of the rows of the level and of the dense inverse; the
+/// eight lanes that sum a row hand its value to the eight blocks, and a
+/// cluster barrier ends each product.  In one block the products were its
+/// 11 us: some 20k entries of three shared-memory words each, read with the
+/// conflicts of ragged rows.  Cluster q works on vector q and does nothing
+/// when done[q] is set (done may be null).
+__global__ void __launch_bounds__(kTailThreads) __cluster_dims__(kTailBlocks, 1, 1)
+k_amg_tail(const int* __restrict__ done, TailLevel T)
+{
+    pdl_entry();
+    const int q = blockIdx.x / kTailBlocks, rank = blockIdx.x % kTailBlocks;
+    if (done && done[q]) return;
+    clusterArrive();  // waited for before the first value goes to another block
+    extern __shared__ __align__(16) int tsm[];
+    const int n = T.n, nc = T.nc, t = threadIdx.x;
+    const int lo = tailFirst(n, rank), rows = tailFirst(n, rank + 1) - lo;
+    const int lod = tailFirst(nc, rank), rowsd = tailFirst(nc, rank + 1) - lod;
+    int* rs = tsm;
+    int* cols = rs + tailShare(n) + 1;
+    float* val = reinterpret_cast<float*>(cols + T.nnz);
+    float* dense = val + T.nnz;
+    float* dinv = dense + tailShare(nc) * nc;
+    int* agg = reinterpret_cast<int*>(dinv + n);
+    int* mem = agg + n;
+    int* ms = mem + n;
+    float* b = reinterpret_cast<float*>(ms + nc + 1);
+    float* x = b + n;
+    float* r = x + n;
+    float* bc = r + n;
+    float* xc = bc + nc;
+    // every copy is under way before the first is waited for
+    auto copy = [&](void* to, const void* from, int words) {
+        const unsigned at = static_cast<unsigned>(__cvta_generic_to_shared(to));
+        for (int i = t; i < words; i += kTailThreads) copyWord(at + 4u * static_cast<unsigned>(i), static_cast<const int*>(from) + i);
+    };
+    const int e0 = T.rs[lo], entries = T.rs[lo + rows] - e0;
+    copy(dinv, T.dinv, n);
+    copy(agg, T.agg, n);
+    copy(mem, T.mem, n);
+    copy(ms, T.ms, nc + 1);
+    copy(rs, T.rs + lo, rows + 1);
+    copy(dense, T.dense + static_cast<size_t>(lod) * nc, rowsd * nc);
+    for (int i = t; i < n; i += kTailThreads)
+        copyWord(static_cast<unsigned>(__cvta_generic_to_shared(b + i)), T.b + static_cast<size_t>(i) * T.stride + q);
+    copy(val, T.val + e0, entries);
+    copy(cols, T.cols + e0, entries);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    for (int i = t; i < n; i += kTailThreads) x[i] = T.w.w[0] * dinv[i] * b[i];  // its own copies
+    __syncthreads();
+    clusterWait();
+    const int l = t % kTailLanes, mine = t / kTailLanes;  // the group's row of the share, its aggregate
+    // every lane: (A v) of the group's row
+    auto product = [&](const float* v) {
+        float s = 0.0f;
+        if (mine < rows)
+            for (int e = rs[mine] - e0 + l; e < rs[mine + 1] - e0; e += kTailLanes) s += val[e] * v[cols[e]];
+#pragma unroll
+        for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        return s;
+    };
+    const int i = lo + mine;  // the group's row
+    // out = f((A in)_i) in every block
+    auto pass = [&](const float* in, float* out, auto f) {
+        const float s = product(in);
+        if (mine < rows) putAt(out + i, l, f(s));
+        clusterArrive();
+        clusterWait();
+    };
+    float *u = x, *v = r;
+    auto sweep = [&](float w) {
+        pass(u, v, [&](float s) { return u[i] + w * dinv[i] * (b[i] - s); });
+        float* const c = u;
+        u = v;
+        v = c;
+    };
+    for (int k = 1; k < T.w.m; ++k) sweep(T.w.w[k]);
+    pass(u, v, [&](float s) { return b[i] - s; });
+    // restriction, in every block
+    {
+        float s = 0.0f;
+        if (mine < nc)
+            for (int k = ms[mine] + l; k < ms[mine + 1]; k += kTailLanes) s += v[mem[k]];
+#pragma unroll
+        for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (mine < nc && l == 0) bc[mine] = s;
+    }
+    __syncthreads();
+    // the coarsest solve xc = M bc: a warp per row of the share
+    {
+        const int lane = t & 31;
+        for (int d = t >> 5; d < rowsd; d += kTailThreads / 32)
+        {
+            float s = 0.0f;
+            for (int j = lane; j < nc; j += 32) s += dense[d * nc + j] * bc[j];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane < kTailBlocks) putAt(xc + lod + d, lane, s);
+        }
+    }
+    clusterArrive();
+    clusterWait();
+    for (int k = t; k < n; k += kTailThreads) u[k] = u[k] + T.scale * xc[agg[k]];
+    __syncthreads();
+    for (int k = T.w.m - 1; k > 0; --k) sweep(T.w.w[k]);
+    const float s = product(u);
+    if (mine < rows && l == 0) T.o[static_cast<size_t>(i) * T.stride + q] = u[i] + T.w.w[0] * dinv[i] * (b[i] - s);
+}
+
+constexpr int kTailBlockLanes = 4;
+
+/// Shared-memory layout of k_amg_tail_block (4-byte words): the level's CSR
 /// (rs n + 1, cols nnz, val nnz), dinv n, agg n, the aggregates' member
 /// lists (ms nc + 1, mem n), the dense inverse nc * nc, the vectors b, x, r
 /// n each, bc and xc nc each.
-__host__ __device__ constexpr size_t tailSmemWords(int n, int nnz, int nc)
+__host__ __device__ constexpr size_t tailBlockWords(int n, int nnz, int nc)
 {
     return static_cast<size_t>(n + 1) + 2 * static_cast<size_t>(nnz) + 2 * static_cast<size_t>(n) +
            static_cast<size_t>(nc + 1) + static_cast<size_t>(n) + static_cast<size_t>(nc) * nc + 3 * static_cast<size_t>(n) +
            2 * static_cast<size_t>(nc);
 }
 
-/// The last aggregation level (at most kTailMax rows) and the coarsest solve
-/// in one block per vector, the level held in shared memory: one coalesced
+/// The same for a small level (kTailClusterEntries): the last aggregation
+/// level and the coarsest solve in one block per vector, the level held in shared memory: one coalesced
 /// load of its matrix, aggregates, dense inverse and right-hand side, then
 /// the sweeps and the residual, restriction, dense solve, prolongation and
 /// the sweeps again, separated by block barriers.  Block q works on vector q
 /// and does nothing when done[q] is set (done may be null); only the output
 /// goes back to global memory.
-__global__ void __launch_bounds__(kTailThreads) k_amg_tail(const int* __restrict__ done, TailLevel T)
+__global__ void __launch_bounds__(kTailThreads) k_amg_tail_block(const int* __restrict__ done, TailLevel T)
 {
     pdl_entry();
     const int q = blockIdx.x;
@@ -795,19 +951,19 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(const int* __restrict
     for (int i = t; i <= nc; i += kTailThreads) ms[i] = T.ms[i];
     for (int i = t; i < nc * nc; i += kTailThreads) dense[i] = T.dense[i];
     __syncthreads();
-    const int l = t % kTailLanes, first = t / kTailLanes, stride = kTailThreads / kTailLanes;
+    const int l = t % kTailBlockLanes, first = t / kTailBlockLanes, stride = kTailThreads / kTailBlockLanes;
     // out(i, (A v)_i) for every row, a group of lanes per row
     auto product = [&](const float* v, auto out) {
         for (int i0 = first;; i0 += stride)
         {
-            const int base = i0 - (t % 32) / kTailLanes;
+            const int base = i0 - (t % 32) / kTailBlockLanes;
             if (base >= n) break;
             const int i = i0 < n ? i0 : -1;
             float s = 0.0f;
             if (i >= 0)
-                for (int e = rs[i] + l; e < rs[i + 1]; e += kTailLanes) s += val[e] * v[cols[e]];
+                for (int e = rs[i] + l; e < rs[i + 1]; e += kTailBlockLanes) s += val[e] * v[cols[e]];
 #pragma unroll
-            for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            for (int o = kTailBlockLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
             if (i >= 0 && l == 0) out(i, s);
         }
         __syncthreads();
@@ -825,14 +981,14 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail(const int* __restrict
     // restriction
     for (int I0 = first;; I0 += stride)
     {
-        const int base = I0 - (t % 32) / kTailLanes;
+        const int base = I0 - (t % 32) / kTailBlockLanes;
         if (base >= nc) break;
         const int I = I0 < nc ? I0 : -1;
         float s = 0.0f;
         if (I >= 0)
-            for (int k = ms[I] + l; k < ms[I + 1]; k += kTailLanes) s += v[mem[k]];
+            for (int k = ms[I] + l; k < ms[I + 1]; k += kTailBlockLanes) s += v[mem[k]];
 #pragma unroll
-        for (int o = kTailLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        for (int o = kTailBlockLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
         if (I >= 0 && l == 0) bc[I] = s;
     }
     __syncthreads();
@@ -1138,12 +1294,21 @@ void Ctx::amgSetup(AmgUse use, const double* vals, double theta)
             if (l >= 1) V.gRow = pick(static_cast<double>(a->lv[l - 1].nnzNext) / V.n, V.n);
         }
     }
-    // the tail level's shared-memory copy, when it and the dense inverse fit
-    // in one block's opt-in shared memory (set before any stream capture)
+    // the tail level's shared-memory copy, when a block's part fits in its
+    // opt-in shared memory (set before any stream capture)
     if (const int T = static_cast<int>(a->lv.size()) - 2; T >= 1 && a->lv[static_cast<size_t>(T)].n <= kTailMax)
     {
-        const int nnz = a->lv[static_cast<size_t>(T) - 1].nnzNext;
-        const size_t bytes = 4 * tailSmemWords(a->lv[T].n, nnz, a->lv[static_cast<size_t>(T) + 1].n);
+        const int n = a->lv[static_cast<size_t>(T)].n;
+        std::vector<int> rs(static_cast<size_t>(n) + 1);
+        CFG_CUDA(cudaMemcpyAsync(rs.data(), a->lv[static_cast<size_t>(T)].rs, rs.size() * sizeof(int), cudaMemcpyDeviceToHost, stream_));
+        CFG_CUDA(cudaStreamSynchronize(stream_));
+        int nnz = 0;
+        for (int k = 0; k < kTailBlocks; ++k)
+            nnz = std::max(nnz, rs[static_cast<size_t>(tailFirst(n, k + 1))] - rs[static_cast<size_t>(tailFirst(n, k))]);
+        const int nc = a->lv[static_cast<size_t>(T) + 1].n, all = rs[static_cast<size_t>(n)];
+        a->tailCluster = all > kTailClusterEntries;
+        if (!a->tailCluster) nnz = all;
+        const size_t bytes = 4 * (a->tailCluster ? tailSmemWords(n, nnz, nc) : tailBlockWords(n, nnz, nc));
         int optin = 0;
         CFG_CUDA(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
         if (bytes <= static_cast<size_t>(optin))
@@ -1157,8 +1322,8 @@ void Ctx::amgSetup(AmgUse use, const double* vals, double theta)
                                    [&](const std::pair<int, size_t>& g) { return g.first == device_; });
             if (it == granted.end() || it->second < bytes)
             {
-                CFG_CUDA(cudaFuncSetAttribute(k_amg_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                              static_cast<int>(bytes)));
+                for (const auto kernel : {k_amg_tail, k_amg_tail_block})
+                    CFG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)));
                 if (it == granted.end()) granted.push_back({device_, bytes});
                 else it->second = bytes;
             }
@@ -1417,7 +1582,8 @@ void coarseCycle(const AmgState& a, bool pdl, int sms, cudaStream_t stream, cons
         t.stride = stride;
         t.scale = scale;
         t.w = sm.at(last);
-        launchK(pdl, k_amg_tail, vectors, kTailThreads, a.tailSmem, stream, stop, t);
+        if (a.tailCluster) launchK(pdl, k_amg_tail, vectors * kTailBlocks, kTailThreads, a.tailSmem, stream, stop, t);
+        else launchK(pdl, k_amg_tail_block, vectors, kTailThreads, a.tailSmem, stream, stop, t);
     }
     else
         launchK(pdl, k_amg_dense, vectors, kDenseMax, 0, stream, stop, a.nc, stride, a.dense,
