@@ -235,8 +235,8 @@ __device__ __forceinline__ float sell_row(const DMat& A, const float* __restrict
 
 /// finest level, first sweep and residual: x = w D^-1 b, r = b - A x
 template <int W>
-__global__ void __launch_bounds__(TPB) k_amg_pre0(const int* __restrict__ stop, DMat A, const float* __restrict__ val,
-                                                  const float* __restrict__ dinv, const double* __restrict__ b,
+__global__ void __launch_bounds__(TPB) k_amg_pre0(const int* stop, DMat A, const float* __restrict__ val,
+                                                  const float* __restrict__ dinv, const double* b,
                                                   float* __restrict__ x, float* __restrict__ r)
 {
     pdl_entry();
@@ -246,7 +246,7 @@ __global__ void __launch_bounds__(TPB) k_amg_pre0(const int* __restrict__ stop, 
         const float bc = static_cast<float>(b[c]);
         x[c] = kOmega * dinv[c] * bc;
         const float s =
-            sell_row<W>(A, val, c, [&](int j) { return kOmega * __ldg(dinv + j) * static_cast<float>(__ldg(b + j)); });
+            sell_row<W>(A, val, c, [&](int j) { return kOmega * __ldg(dinv + j) * static_cast<float>(b[j]); });
         r[c] = bc - s;
     }
 }
@@ -255,10 +255,10 @@ __global__ void __launch_bounds__(TPB) k_amg_pre0(const int* __restrict__ stop, 
 /// FCG (st given) also z.q and, in the block that finishes last,
 /// beta = -z.q / p.q
 template <int W>
-__global__ void __launch_bounds__(TPB) k_amg_post0(const int* __restrict__ stop, DMat A, const float* __restrict__ val,
-                                                   const float* __restrict__ dinv, const double* __restrict__ b,
-                                                   const float* __restrict__ y, double* __restrict__ z,
-                                                   const double* __restrict__ q, double* partials, FcgState* st)
+__global__ void __launch_bounds__(TPB) k_amg_post0(const int* stop, DMat A, const float* __restrict__ val,
+                                                   const float* __restrict__ dinv, const double* b, const float* y,
+                                                   double* __restrict__ z, const double* q, double* partials,
+                                                   FcgState* st)
 {
     pdl_entry();
     if (stop && *stop) return;
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(TPB) k_amg_post0(const int* __restrict__ stop,
     double zq[1] = {0.0};
     FOR_ROWS(c, A.n)
     {
-        const float s = sell_row<W>(A, val, c, [&](int j) { return __ldg(y + j); });
+        const float s = sell_row<W>(A, val, c, [&](int j) { return y[j]; });
         const double zc = static_cast<double>(y[c] + kOmega * dinv[c] * (static_cast<float>(b[c]) - s));
         z[c] = zc;
         if (dot) zq[0] += zc * q[c];
@@ -438,7 +438,7 @@ __device__ __forceinline__ void unpack3(float4 p, float (&v)[3])
 /// finest level, first sweep and residual for three FP64 right-hand sides:
 /// x = w D^-1 b and r = b - A x
 template <int W>
-__global__ void __launch_bounds__(TPB, (W > 0 && W <= 8) ? 6 : 1) k_amgv_pre0(const int* __restrict__ done, DMat A, const float* __restrict__ val,
+__global__ void __launch_bounds__(TPB, (W > 0 && W <= 8) ? 6 : 1) k_amgv_pre0(const int* done, DMat A, const float* __restrict__ val,
                                                    const float* __restrict__ dinv, CV3P b, float4* __restrict__ x,
                                                    float4* __restrict__ r)
 {
@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(TPB, (W > 0 && W <= 8) ? 6 : 1) k_amgv_pre0(co
         sell_row3<W>(A, val, c, s, [&](int j, float (&g)[3]) {
             const float wd = kOmega * __ldg(dinv + j);
 #pragma unroll
-            for (int q = 0; q < 3; ++q) g[q] = act.a[q] ? wd * static_cast<float>(__ldg(b.c[q] + j)) : 0.0f;
+            for (int q = 0; q < 3; ++q) g[q] = act.a[q] ? wd * static_cast<float>(b.c[q][j]) : 0.0f;
         });
         const float dc = dinv[c];
         float xv[3], rv[3];
@@ -470,8 +470,8 @@ __global__ void __launch_bounds__(TPB, (W > 0 && W <= 8) ? 6 : 1) k_amgv_pre0(co
 
 /// finest level: z = y + w D^-1 (b - A y), into FP64 (active components only)
 template <int W>
-__global__ void __launch_bounds__(TPB) k_amgv_post0(const int* __restrict__ done, DMat A, const float* __restrict__ val,
-                                                    const float* __restrict__ dinv, CV3P b, const float4* __restrict__ y,
+__global__ void __launch_bounds__(TPB) k_amgv_post0(const int* done, DMat A, const float* __restrict__ val,
+                                                    const float* __restrict__ dinv, CV3P b, const float4* y,
                                                     V3P z)
 {
     pdl_entry();
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(TPB) k_amgv_post0(const int* __restrict__ done
     FOR_ROWS(c, n)
     {
         float s[3];
-        sell_row3<W>(A, val, c, s, [&](int j, float (&g)[3]) { unpack3(__ldg(y + j), g); });
+        sell_row3<W>(A, val, c, s, [&](int j, float (&g)[3]) { unpack3(y[j], g); });
         const float dc = dinv[c];
         float yc[3];
         unpack3(y[c], yc);
@@ -554,10 +554,7 @@ __device__ __forceinline__ V group_row(const Coarse<V>& L, int i, int l, const V
     vzero(s);
     if (i >= 0)
         for (int e = __ldg(L.rs + i) + l; e < __ldg(L.rs + i + 1); e += G)
-        {
-            const V* p = x + __ldg(L.cols + e);
-            vmad(s, __ldg(L.val + e), __ldg(p));
-        }
+            vmad(s, __ldg(L.val + e), x[__ldg(L.cols + e)]);
     vgroup<G>(s);
     return s;
 }
@@ -586,10 +583,7 @@ __device__ __forceinline__ void do_restrict(int n, const int* __restrict__ ms, c
         vzero(s);
         if (I >= 0)
             for (int k = __ldg(ms + I) + l; k < __ldg(ms + I + 1); k += G)
-            {
-                const V* p = r + __ldg(mem + k);
-                s = vadd(s, __ldg(p));
-            }
+                s = vadd(s, r[__ldg(mem + k)]);
         vgroup<G>(s);
         if (I < 0 || l != 0) return;
         b[I] = s;
@@ -618,8 +612,8 @@ __device__ __forceinline__ void do_smooth(const Coarse<V>& L, float w, const V* 
 }
 
 template <class V, int G>
-__global__ void __launch_bounds__(TPB) k_amg_restrict(const int* __restrict__ stop, int n, const int* __restrict__ ms,
-                                                      const int* __restrict__ mem, const V* __restrict__ r,
+__global__ void __launch_bounds__(TPB) k_amg_restrict(const int* stop, int n, const int* __restrict__ ms,
+                                                      const int* __restrict__ mem, const V* r,
                                                       const float* __restrict__ dinv, float w, V* __restrict__ b,
                                                       V* __restrict__ x)
 {
@@ -629,8 +623,7 @@ __global__ void __launch_bounds__(TPB) k_amg_restrict(const int* __restrict__ st
 }
 
 template <class V, int G>
-__global__ void __launch_bounds__(TPB) k_amg_residual(const int* __restrict__ stop, Coarse<V> L, const V* __restrict__ x,
-                                                      V* __restrict__ r)
+__global__ void __launch_bounds__(TPB) k_amg_residual(const int* stop, Coarse<V> L, const V* x, V* __restrict__ r)
 {
     pdl_entry();
     if (halted(stop, V{})) return;
@@ -638,8 +631,7 @@ __global__ void __launch_bounds__(TPB) k_amg_residual(const int* __restrict__ st
 }
 
 template <class V, int G>
-__global__ void __launch_bounds__(TPB) k_amg_smooth(const int* __restrict__ stop, Coarse<V> L, float w, const V* __restrict__ y,
-                                                    V* __restrict__ out)
+__global__ void __launch_bounds__(TPB) k_amg_smooth(const int* stop, Coarse<V> L, float w, const V* y, V* __restrict__ out)
 {
     pdl_entry();
     if (halted(stop, V{})) return;
@@ -648,8 +640,7 @@ __global__ void __launch_bounds__(TPB) k_amg_smooth(const int* __restrict__ stop
 
 /// the coarse correction brought to a level: y = x + s P xc
 template <class V>
-__global__ void __launch_bounds__(TPB) k_amg_prolong(const int* __restrict__ stop, int n, const V* __restrict__ x,
-                                                     const V* __restrict__ xc, const int* __restrict__ agg,
+__global__ void __launch_bounds__(TPB) k_amg_prolong(const int* stop, int n, const V* x, const V* xc, const int* __restrict__ agg,
                                                      V* __restrict__ y, float scale)
 {
     pdl_entry();
@@ -669,7 +660,7 @@ __global__ void __launch_bounds__(TPB) k_amg_to_sell(int nnz, const int* __restr
 }
 
 template <class V>
-__device__ __forceinline__ V sell32_row(const Coarse<V>& L, int i, const V* __restrict__ x)
+__device__ __forceinline__ V sell32_row(const Coarse<V>& L, int i, const V* x)
 {
     const int e0 = __ldg(L.sstart + (i >> 5)) + (i & 31), e1 = __ldg(L.sstart + (i >> 5) + 1);
     V s;
@@ -689,7 +680,7 @@ __device__ __forceinline__ V sell32_row(const Coarse<V>& L, int i, const V* __re
 #pragma unroll
         for (int k = 0; k < 8; ++k)
         {
-            if (col[k] >= 0) g[k] = __ldg(x + col[k]);
+            if (col[k] >= 0) g[k] = x[col[k]];
             else vzero(g[k]);
         }
 #pragma unroll
@@ -700,8 +691,7 @@ __device__ __forceinline__ V sell32_row(const Coarse<V>& L, int i, const V* __re
 
 /// r = b - A x
 template <class V>
-__global__ void __launch_bounds__(TPB) k_amg_residual_sell(const int* __restrict__ stop, Coarse<V> L,
-                                                           const V* __restrict__ x, V* __restrict__ r)
+__global__ void __launch_bounds__(TPB) k_amg_residual_sell(const int* stop, Coarse<V> L, const V* x, V* __restrict__ r)
 {
     pdl_entry();
     if (halted(stop, V{})) return;
@@ -710,8 +700,7 @@ __global__ void __launch_bounds__(TPB) k_amg_residual_sell(const int* __restrict
 
 /// out = y + w D^-1 (b - A y)
 template <class V>
-__global__ void __launch_bounds__(TPB) k_amg_smooth_sell(const int* __restrict__ stop, Coarse<V> L, float w,
-                                                         const V* __restrict__ y, V* __restrict__ out)
+__global__ void __launch_bounds__(TPB) k_amg_smooth_sell(const int* stop, Coarse<V> L, float w, const V* y, V* __restrict__ out)
 {
     pdl_entry();
     if (halted(stop, V{})) return;
@@ -792,7 +781,7 @@ __device__ __forceinline__ void clusterWait() { asm volatile("barrier.cluster.wa
 /// conflicts of ragged rows.  Cluster q works on vector q and does nothing
 /// when done[q] is set (done may be null).
 __global__ void __launch_bounds__(kTailThreads) __cluster_dims__(kTailBlocks, 1, 1)
-k_amg_tail(const int* __restrict__ done, TailLevel T)
+k_amg_tail(const int* done, TailLevel T)
 {
     pdl_entry();
     const int q = blockIdx.x / kTailBlocks, rank = blockIdx.x % kTailBlocks;
@@ -913,7 +902,7 @@ __host__ __device__ constexpr size_t tailBlockWords(int n, int nnz, int nc)
 /// the sweeps again, separated by block barriers.  Block q works on vector q
 /// and does nothing when done[q] is set (done may be null); only the output
 /// goes back to global memory.
-__global__ void __launch_bounds__(kTailThreads) k_amg_tail_block(const int* __restrict__ done, TailLevel T)
+__global__ void __launch_bounds__(kTailThreads) k_amg_tail_block(const int* done, TailLevel T)
 {
     pdl_entry();
     const int q = blockIdx.x;
@@ -1023,8 +1012,8 @@ __global__ void __launch_bounds__(kTailThreads) k_amg_tail_block(const int* __re
 
 /// the coarsest solve x = M b with the dense inverse, when the tail kernel
 /// does not hold the level above it (block q: vector q)
-__global__ void __launch_bounds__(kDenseMax) k_amg_dense(const int* __restrict__ done, int n, int stride,
-                                                         const float* __restrict__ m, const float* __restrict__ b,
+__global__ void __launch_bounds__(kDenseMax) k_amg_dense(const int* done, int n, int stride,
+                                                         const float* __restrict__ m, const float* b,
                                                          float* __restrict__ x)
 {
     pdl_entry();
@@ -1773,9 +1762,8 @@ __global__ void __launch_bounds__(TPB) k_fcgd_init(DMat A, const double* __restr
 /// old p stays for the other rows, the new one goes to pNew); beta is 0 in
 /// the first iteration and p zero.
 template <int W, bool kForm>
-__global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restrict__ val, const double* __restrict__ z,
-                                                   const double* __restrict__ p, double* __restrict__ pNew,
-                                                   const double* __restrict__ r, double* __restrict__ q,
+__global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restrict__ val, const double* z, const double* p,
+                                                   double* __restrict__ pNew, const double* r, double* __restrict__ q,
                                                    double* partials, FcgState* st)
 {
     pdl_entry();
@@ -1786,7 +1774,7 @@ __global__ void __launch_bounds__(TPB) k_fcgd_spmv(DMat A, const double* __restr
     {
         double y[1];
         spmv_row_gather<W, 1>(A, val, c, y, [&](int col, double (&xv)[1]) {
-            xv[0] = kForm ? __ldg(z + col) + be * __ldg(p + col) : __ldg(p + col);
+            xv[0] = kForm ? z[col] + be * p[col] : p[col];
         });
         q[c] = y[0];
         const double pc = kForm ? z[c] + be * p[c] : p[c];
@@ -1844,7 +1832,7 @@ __device__ __forceinline__ void fcg_update_end(double (&s)[1], bool inf, double*
 }
 
 /// x += alpha p, r -= alpha q, |r| and the stopping test
-__global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* __restrict__ p, const double* __restrict__ q,
+__global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* p, const double* q,
                                                      double* __restrict__ x, double* __restrict__ r, double* partials,
                                                      FcgState* st)
 {
@@ -1864,7 +1852,7 @@ __global__ void __launch_bounds__(TPB) k_fcgd_update(int n, const double* __rest
 }
 
 /// p = z + beta p
-__global__ void __launch_bounds__(TPB) k_fcgd_p(int n, const double* __restrict__ z, double* __restrict__ p,
+__global__ void __launch_bounds__(TPB) k_fcgd_p(int n, const double* z, double* __restrict__ p,
                                                 const FcgState* st)
 {
     pdl_entry();
@@ -1879,9 +1867,8 @@ __global__ void __launch_bounds__(TPB) k_fcgd_p(int n, const double* __restrict_
 /// rows).  When the test is met the sweep has been for nothing, once a solve.
 template <int W>
 __global__ void __launch_bounds__(TPB) k_fcgd_update_pre0(DMat A, const float* __restrict__ val,
-                                                          const float* __restrict__ dinv, const double* __restrict__ p,
-                                                          const double* __restrict__ q, double* __restrict__ x,
-                                                          const double* __restrict__ r, double* __restrict__ rNew,
+                                                          const float* __restrict__ dinv, const double* p, const double* q,
+                                                          double* __restrict__ x, const double* r, double* __restrict__ rNew,
                                                           float* __restrict__ xs, float* __restrict__ rs,
                                                           double* partials, FcgState* st)
 {
@@ -1894,7 +1881,7 @@ __global__ void __launch_bounds__(TPB) k_fcgd_update_pre0(DMat A, const float* _
     {
         const double rc = r[c] - al * q[c];
         const float sum = sell_row<W>(A, val, c, [&](int j) {
-            return kOmega * __ldg(dinv + j) * static_cast<float>(__ldg(r + j) - al * __ldg(q + j));
+            return kOmega * __ldg(dinv + j) * static_cast<float>(r[j] - al * q[j]);
         });
         const float bc = static_cast<float>(rc);
         x[c] = x[c] + al * p[c];

@@ -434,10 +434,10 @@ private:
     // 3.02 -> 2.88 ms, 158k-cell PISO step 8.33 -> 7.96 ms); above, the
     // waiting blocks hold the running kernel's slots (262k cells 42.6 -> 43.3
     // ms, 2M 298 -> 302 ms before the sweeps' change).  CHUANFLOW_PDL=1: on
-    // every size.  The results are the same.
+    // every size, 0: on none.  The results are the same.
     static constexpr int kPdlRows = 200000;
-    bool amgPdl() const { return pdl_ || dm_.nC <= kPdlRows; }
-    bool pdl_ = false;
+    bool amgPdl() const { return pdl_ < 0 ? dm_.nC <= kPdlRows : pdl_ != 0; }
+    int pdl_ = -1;  // CHUANFLOW_PDL; -1: not set
     std::map<std::string, cudaGraphExec_t> graphs_;
     static constexpr int kEvPerIter = 12;  // events per solver iteration of a chunk (timed segments + 1)
     std::vector<cudaEvent_t> kev_;

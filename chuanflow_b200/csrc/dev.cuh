@@ -16,6 +16,13 @@ namespace cfg
 /// is that of plain stream order; what overlaps is the launch and block
 /// scheduling of one kernel with the tail of the one before.  Both
 /// instructions are no-ops for a kernel launched without the attribute.
+///
+/// Such a kernel reads what other kernels of its chain write (vectors, flags,
+/// scalars) with ordinary loads only: no __ldg and no const __restrict__
+/// pointer.  The read-only path asks for data that stay as they are for the
+/// kernel's whole life, which here begins while its predecessors still write;
+/// its loads may also be moved above the wait.  Matrix values, patterns,
+/// aggregates and D^-1 are complete before a chain begins and may take it.
 __device__ __forceinline__ void pdl_entry()
 {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");

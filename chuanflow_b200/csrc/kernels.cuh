@@ -330,7 +330,10 @@ __global__ void __launch_bounds__(TPB) k_grad_ls2(DMesh m, CV3P x, BcTab bc, CGr
 /// independent loads in flight instead of walking a dependent chain.  W = 0
 /// walks rows of any length.  Entries are added in order, skipping only the
 /// trailing pads, so the sum is the reference's.  T = float forms each
-/// product in single precision and accumulates in double.
+/// product in single precision and accumulates in double.  x is read with
+/// ordinary loads: some callers are programmatic dependents of the kernel
+/// that writes it (pdl_entry); a caller whose x is const __restrict__ gets
+/// read-only loads from the compiler.
 template <int W, int NC, class T = double>
 __device__ __forceinline__ void spmv_row(const DMat& A, const T* __restrict__ val, int c, const T* const (&x)[NC],
                                          double (&y)[NC])
@@ -359,7 +362,7 @@ __device__ __forceinline__ void spmv_row(const DMat& A, const T* __restrict__ va
 #pragma unroll
             for (int k = 0; k < CH; ++k)
 #pragma unroll
-                for (int q = 0; q < NC; ++q) xv[q][k] = col[k] >= 0 ? __ldg(x[q] + col[k]) : T(0);
+                for (int q = 0; q < NC; ++q) xv[q][k] = col[k] >= 0 ? x[q][col[k]] : T(0);
 #pragma unroll
             for (int k = 0; k < CH; ++k)
                 if (col[k] >= 0)

@@ -686,7 +686,7 @@ void Ctx::buildDevice()
     G_ = std::max(1, std::min((nC + TPB - 1) / TPB, sms * 8));
     sms_ = sms;
     if (const char* e = std::getenv("CHUANFLOW_ROW_BLOCKS_PER_SM")) rowBlocksPerSM_ = std::max(0, std::atoi(e));
-    if (const char* e = std::getenv("CHUANFLOW_PDL")) pdl_ = std::atoi(e) != 0;
+    if (const char* e = std::getenv("CHUANFLOW_PDL")) pdl_ = std::atoi(e) != 0 ? 1 : 0;
     GS_ = rowGrid(nC);
     initRowBlocks_ = rowBlocksPerSM_;
     initGS_ = GS_;
