@@ -530,6 +530,11 @@ int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32
     });
 }
 
+int cfg_solver_wait_limit(int64_t cycles)
+{
+    return guard([&] { cfg::setTeamWaitLimit(cycles); });
+}
+
 int cfg_amg_strength(cfg_ctx* ctx, double theta)
 {
     return guard([&] {

@@ -28,6 +28,10 @@ struct TeamPlan
 };
 TeamPlan teamPlanOf(int n, int nComp, int clusterMax, int sms, bool gridOk);
 int largestCluster(int device);
+/// GPU cycles after which a wait inside a grid team gives up, for the solves
+/// the calling thread starts (cfg_solver_wait_limit).
+long long teamWaitLimit();
+void setTeamWaitLimit(long long cycles);
 
 struct Timing
 {
@@ -221,7 +225,7 @@ private:
     void teamCg(const TeamPlan& tp, const double* vals, const double* diag, const double* b, double* x,
                 const double* rDinv, double tol, int maxIter, int normType);
     void teamReport(int nComp, cfg_solver_report* reps);
-    void checkTeam() const;
+    void checkTeam();
     int clusterMax_ = 0;            // largest cluster this device runs
     bool coopOk_ = false;           // cooperative launches
     int* dColour_ = nullptr;        // DIC colour of each row

@@ -476,7 +476,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
     for (int k = 0; k < K; ++k)
     {
         const int i = threadIdx.x + k * kTeamThreads;
-        if (i < cnt && sc.fits) a.x[lo + i] = x[k];
+        if (i < cnt && !tm.dead() && sc.fits) a.x[lo + i] = x[k];
     }
     if (tm.rank == 0 && threadIdx.x == 0)
     {
@@ -756,7 +756,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_bicg(PersBi<Mat> a, Pe
     for (int k = 0; k < K; ++k)
     {
         const int i = threadIdx.x + k * kTeamThreads;
-        if (i < cnt)
+        if (i < cnt && !tm.dead())
 #pragma unroll
             for (int q = 0; q < NC; ++q) a.x.c[q0 + q][lo + i] = X(k, q);
     }
@@ -809,7 +809,8 @@ void dispatchK(int K, F&& f)
 
 inline TeamMem teamMem(const TeamPlan& tp, int n, unsigned* count, double* part, int* failed)
 {
-    return TeamMem{tp.blocks, count, part, (n + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, failed};
+    return TeamMem{tp.blocks, count, part, (n + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, failed,
+                   teamWaitLimit()};
 }
 /// doubles of `part` for a system of n rows in one team, and in any plan
 constexpr size_t teamPartMax(int n) { return 2 * kTeamVals * (static_cast<size_t>(n) / kGroupRows + 1); }

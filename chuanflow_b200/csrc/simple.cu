@@ -635,6 +635,13 @@ Ctx::~Ctx()
     if (ownStream_) cudaStreamDestroy(stream_);
 }
 
+namespace
+{
+thread_local long long g_teamWait = kTeamWaitCycles;
+}
+long long teamWaitLimit() { return g_teamWait; }
+void setTeamWaitLimit(long long cycles) { g_teamWait = cycles > 0 ? cycles : kTeamWaitCycles; }
+
 /// The largest cluster of whole-solve blocks the device runs: 16 (a
 /// non-portable size, which a partitioned GPU may not have), else 8, else 0.
 int largestCluster(int device)
@@ -1571,10 +1578,14 @@ void Ctx::teamReport(int nComp, cfg_solver_report* reps)
     }
 }
 
-void Ctx::checkTeam() const
+/// Reports a wait that ran out, once: the kernel left its counters ready, so
+/// the context's next solve starts clean.
+void Ctx::checkTeam()
 {
-    if (*static_cast<volatile int*>(teamFailed_))
-        fail(CFG_ECUDA, "solver: a wait inside a kernel ran out");
+    volatile int* const flag = teamFailed_;
+    if (!*flag) return;
+    *flag = 0;
+    fail(CFG_ECUDA, "solver: a wait inside a kernel ran out");
 }
 
 void Ctx::runCG(const double* vals, const double* diag, const double* b, double* x, double tol, int maxIter,

@@ -74,9 +74,14 @@ bool residentSolve(int device, int n, int maxRow, const int64_t* rs, const int64
         bytes += (size + 255) / 256 * 256;
         return at;
     };
-    // the zeroed part first: counters, the failure flag and the state
-    const size_t oCount = place(kTeamsMax * kCountStride * sizeof(unsigned)), oFail = place(sizeof(int)),
-                 oState = place(sizeof(SolveState)), zeroed = bytes;
+    // the zeroed part first: counters, the state and the failure flag
+    struct Outcome
+    {
+        SolveState st;
+        int failed;
+    };
+    const size_t oCount = place(kTeamsMax * kCountStride * sizeof(unsigned)), oOutcome = place(sizeof(Outcome)),
+                 zeroed = bytes;
     const size_t oRs = place((N + 1) * sizeof(int64_t)), oCols = place(nnz * sizeof(int64_t)),
                  oVals = place(nnz * sizeof(double)), oB = place(N * sizeof(double)), oX = place(N * sizeof(double)),
                  oG = place(N * sizeof(double)), oPart = place(teamPartSize(n) * sizeof(double));
@@ -111,10 +116,10 @@ bool residentSolve(int device, int n, int maxRow, const int64_t* rs, const int64
     double* const db = reinterpret_cast<double*>(d + oB);
     double* const dx = reinterpret_cast<double*>(d + oX);
     double* const dg = reinterpret_cast<double*>(d + oG);
-    SolveState* const st = reinterpret_cast<SolveState*>(d + oState);
-    const PersArgs t{tol, maxIter, 0, tp.chunk, st, nullptr,
+    Outcome* const out = reinterpret_cast<Outcome*>(d + oOutcome);
+    const PersArgs t{tol, maxIter, 0, tp.chunk, &out->st, nullptr,
                      teamMem(tp, n, reinterpret_cast<unsigned*>(d + oCount), reinterpret_cast<double*>(d + oPart),
-                             reinterpret_cast<int*>(d + oFail))};
+                             &out->failed)};
     dispatchK<kRes1K>(tp.K, [&](auto Kc) {
         constexpr int K = decltype(Kc)::value;
         if (method == CFG_SOLVE_CG)
@@ -132,13 +137,14 @@ bool residentSolve(int device, int n, int maxRow, const int64_t* rs, const int64
             else launchTeam(tp, 1, k_pers_bicg<K, GridTeam, 1, View>, a, t, smem, s);
         }
     });
-    SolveState h;
-    int failed = 0;
-    CFG_CUDA(cudaMemcpyAsync(&h, st, sizeof h, cudaMemcpyDeviceToHost, s));
-    CFG_CUDA(cudaMemcpyAsync(&failed, d + oFail, sizeof failed, cudaMemcpyDeviceToHost, s));
+    // the caller's x changes only once the solve is known to have ended well
+    Outcome got;
+    CFG_CUDA(cudaMemcpyAsync(&got, out, sizeof got, cudaMemcpyDeviceToHost, s));
+    CFG_CUDA(cudaStreamSynchronize(s));
+    if (got.failed) fail(CFG_ECUDA, "sparse solve: a wait inside a kernel ran out");
     CFG_CUDA(cudaMemcpyAsync(x, dx, N * sizeof(double), cudaMemcpyDeviceToHost, s));
     CFG_CUDA(cudaStreamSynchronize(s));
-    if (failed) fail(CFG_ECUDA, "sparse solve: a wait inside a kernel ran out");
+    const SolveState& h = got.st;
     rep->iterations = h.it[0];
     rep->converged = h.conv[0];
     rep->initial_residual = h.init[0];

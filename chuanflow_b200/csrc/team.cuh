@@ -53,7 +53,8 @@ __device__ __forceinline__ double mag_value(unsigned long long b)
 /// The teams of a launch (one per component of a solve whose components
 /// iterate on their own) and the global-memory side of grid teams: per team
 /// an arrival counter, an exit counter that resets both for the next launch
-/// and two sets of partials; a host-mapped flag raised when a wait ran out.
+/// and two sets of partials; a flag raised when a wait ran out, and the GPU
+/// cycles after which it does.
 constexpr int kTeamsMax = 3;
 constexpr int kCountStride = 64;  // a team's counters on lines of their own
 struct TeamMem
@@ -64,6 +65,7 @@ struct TeamMem
     int groups;        // 256-row groups of the system
     int perBlock;      // and of one block
     int* failed;
+    long long wait;
 };
 
 struct TeamSmem
@@ -282,9 +284,15 @@ struct ClusterTeam
 };
 
 /// A cooperative grid, one block per SM at most.  A wait that has not been
-/// met after kTeamWaitCycles marks the team dead and returns; every body
-/// checks dead() after each sync and reduction and leaves.
+/// met after `wait` cycles marks the block dead and returns; every body checks
+/// dead() after each sync and reduction, leaves without storing its solution
+/// and still counts itself out, so the counters are ready for the next launch.
 constexpr long long kTeamWaitCycles = 4000000000LL;  // about two seconds
+
+/// whether `seen` arrivals have reached `target`, both counted modulo 2^32
+__host__ __device__ constexpr bool arrived(unsigned seen, unsigned target) { return static_cast<int>(seen - target) >= 0; }
+static_assert(arrived(5u, 5u) && !arrived(4u, 5u) && arrived(3u, 0xfffffff0u) && !arrived(0xfffffff0u, 3u),
+              "a count that wraps does not pass its barrier early");
 
 struct GridTeam
 {
@@ -294,19 +302,22 @@ struct GridTeam
     unsigned* count;
     double* part0;
     int* failed;
+    long long wait;
     unsigned target = 0;
     __device__ GridTeam(TeamSmem& s, const TeamMem& g)
         : sm(s), nb(g.blocks), team(blockIdx.x / g.blocks), rank(blockIdx.x % g.blocks), groups(g.groups), per(g.perBlock),
           count(g.count + team * kCountStride), part0(g.part + static_cast<size_t>(team) * 2 * kTeamVals * g.groups),
-          failed(g.failed)
+          failed(g.failed), wait(g.wait)
     {
         if (threadIdx.x == 0) sm.dead = 0;
         __syncthreads();
     }
     __device__ __forceinline__ bool dead() const { return sm.dead != 0; }
-    /// one thread: arrive (after its own writes) and wait for the others
+    /// one thread: arrive (after its own writes) and wait for the others; the
+    /// arrivals are compared by their distance, which a wrapped count keeps
     __device__ __forceinline__ void arrive_wait()
     {
+        if (sm.dead) return;
         __threadfence();
         asm volatile("red.relaxed.gpu.global.add.u32 [%0], 1;" ::"l"(count) : "memory");
         const long long t0 = clock64();
@@ -314,8 +325,8 @@ struct GridTeam
         for (;;)
         {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(count) : "memory");
-            if (seen >= target) break;
-            if (clock64() - t0 > kTeamWaitCycles)
+            if (arrived(seen, target)) break;
+            if (clock64() - t0 > wait)
             {
                 sm.dead = 1;
                 *static_cast<volatile int*>(failed) = 1;

@@ -358,6 +358,14 @@ int cfg_kernel_components(const cfg_ctx* ctx, double* out, int32_t slots);
 int cfg_sparse_solve(const cfg_ctx* ctx_or_null, int32_t device, int64_t n, const int64_t* row_start,
                      const int64_t* cols, const double* vals, const double* b, double* x, double tol,
                      int32_t max_iter, int32_t method, cfg_solver_report* report);
+/* Systems of 32,769 rows and more that fit the GPU's shared memory are solved
+ * by one kernel whose blocks wait for one another between the steps of an
+ * iteration (no counterpart in the reference).  A wait of more than `cycles`
+ * GPU clock cycles (0 or less: the default, about two seconds) ends the solve
+ * with CFG_ECUDA: cfg_sparse_solve leaves the caller's x as it was; a context's
+ * fields are then unspecified until they are set again, and its next solve
+ * starts clean.  Applies to the solves the calling thread starts from now on. */
+int cfg_solver_wait_limit(int64_t cycles);
 
 /* ---- the pressure-Poisson solve on its own (no reference counterpart) ---- */
 
