@@ -4,8 +4,8 @@
 // its rows' matrix entries and the vector its neighbours gather in shared
 // memory and every other vector in registers; an iteration touches global
 // memory only for values a grid team's blocks read from each other.  The
-// arithmetic of each vector element is that of the per-iteration kernels;
-// only the order of the reductions differs.
+// arithmetic of each vector element is that of the per-iteration kernels, and
+// so is the order of the reductions when those run one row per thread.
 #pragma once
 
 #include "dic.cuh"

@@ -37,6 +37,7 @@ constexpr int kTeamRowsMax = 4;  // rows per thread (two partials each per block
 constexpr int kPartMax = 2 * kTeamRowsMax;
 constexpr int kGridFold = 4;     // partials per thread of a grid team's final sum
 constexpr int kGroupsMax = 256 * kGridFold;  // most groups of a system
+static_assert(kGridFold == 4 && kGridFold <= FU, "team_final adds the partials in partial_sum's pairs");
 
 /// Magnitude as an ordered integer: larger magnitudes compare larger and a
 /// NaN above every number, so one integer maximum carries both |v|inf and
@@ -192,9 +193,11 @@ __device__ __forceinline__ void team_final(TeamSmem& sm, int groups, int nb, Sum
 #pragma unroll
             for (int q = 0; q < NS; ++q)
             {
-                double w = t < groups ? a[q][0] : 0.0;
 #pragma unroll
-                for (int k = 1; k < kFold; ++k) w += t + 256 * k < groups ? a[q][k] : 0.0;
+                for (int k = 0; k < kFold; ++k) a[q][k] = t + 256 * k < groups ? a[q][k] : 0.0;
+                // partial_sum's pairs
+                double w = a[q][0];
+                if constexpr (kFold == 4) w = (a[q][0] + a[q][1]) + (a[q][2] + a[q][3]);
                 w = xor_sum<32>(w);
                 if (lane == 0) sm.tree[q][warp] = w;
             }
