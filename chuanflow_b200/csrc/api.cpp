@@ -535,6 +535,11 @@ int cfg_solver_wait_limit(int64_t cycles)
     return guard([&] { cfg::setTeamWaitLimit(cycles); });
 }
 
+int cfg_solver_start_limit(int64_t cycles)
+{
+    return guard([&] { cfg::setTeamStartLimit(cycles); });
+}
+
 int cfg_amg_strength(cfg_ctx* ctx, double theta)
 {
     return guard([&] {

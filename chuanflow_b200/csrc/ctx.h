@@ -32,6 +32,10 @@ int largestCluster(int device);
 /// the calling thread starts (cfg_solver_wait_limit).
 long long teamWaitLimit();
 void setTeamWaitLimit(long long cycles);
+/// and those that the blocks of a plain launch wait for all to be there
+/// (cfg_solver_start_limit)
+long long teamStartLimit();
+void setTeamStartLimit(long long cycles);
 
 struct Timing
 {

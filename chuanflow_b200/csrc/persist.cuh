@@ -26,7 +26,7 @@ struct SellView
     const double* val;
     const double* diag_;
     static constexpr int step = 32;
-    static constexpr bool checked = false;  // rows are known to fit kResW
+    static constexpr bool checked = false;  // every row is known to fit kResW
     __device__ __forceinline__ int n() const { return A.n; }
     __device__ __forceinline__ long long first(int c) const { return __ldg(A.start + (c >> 5)) + (c & 31); }
     __device__ __forceinline__ long long end(int c) const { return __ldg(A.start + (c >> 5) + 1); }
@@ -58,8 +58,10 @@ struct CsrView
 };
 
 /// A solve's arguments beyond its vectors: the stopping test, the rows per
-/// block (contiguous), where the outcome goes, and the optional
-/// {iterations, unconverged} sums of an outer iteration.
+/// block (contiguous), where the outcome goes, the optional {iterations,
+/// unconverged} sums of an outer iteration, and for a matrix whose rows no host
+/// has measured a zero word that is set, with nothing else written, when one
+/// has more than kResW entries.
 struct PersArgs
 {
     double tol;
@@ -69,7 +71,21 @@ struct PersArgs
     SolveState* st;
     double* tally;
     TeamMem g;
+    int* wide = nullptr;
 };
+
+/// whether the team leaves: a row is too long, or a wait ran out (asked first:
+/// then another block may still be writing the word)
+template <class Team, class Mat>
+__device__ __forceinline__ bool too_wide(Team& tm, const Mat& A, int lo, int cnt, int* wide)
+{
+    bool mine = false;
+    for (int i = threadIdx.x; i < cnt; i += kTeamThreads) mine |= A.end(lo + i) - A.first(lo + i) > kResW;
+    volatile int* const w = wide;
+    if (__syncthreads_or(mine) && threadIdx.x == 0) *w = 1;
+    tm.sync();
+    return tm.dead() || *w != 0;
+}
 
 /// whether a solve keeps its matrix entries in registers
 __host__ __device__ constexpr bool resident_regs(int K, int NC, bool jacobiCg) { return NC == 1 && (K == 1 || (K == 2 && jacobiCg)); }
@@ -285,7 +301,7 @@ __device__ __forceinline__ void pers_dic(Team& tm, Res& R, int C, const double (
 struct CgScalars
 {
     double alpha, beta;
-    int go, fits;
+    int go;
 };
 
 /// CG of Matrix.cpp:153-222, preconditioned by D^-1 or the multicolour DIC
@@ -296,6 +312,17 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
     extern __shared__ __align__(16) unsigned char dyn[];
     Team tm(smem, t.g);
     const int n = a.A.n(), lo = min(n, tm.rank * t.chunk), cnt = min(n - lo, t.chunk);
+    if (tm.dead())
+    {
+        tm.finish();
+        return;
+    }
+    if constexpr (Mat::checked)
+        if (t.wide && too_wide(tm, a.A, lo, cnt, t.wide))
+        {
+            tm.finish();
+            return;
+        }
     Resident<K, 1, Team, resident_regs(K, 1, !kDic)> R(dyn, V3P{{a.g, a.g, a.g}}, lo, cnt);
     R.load(a.A, t.chunk, tm.rank);
     const bool two = t.normType != 0;
@@ -341,7 +368,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
     int it = 0, conv = 0;
     {
         double s[K][3];  // r.z, r.r, b.b
-        unsigned long long m[3] = {0, 0, 0};  // |r|, |b|, a row that does not fit
+        unsigned long long m[2] = {0, 0};  // |r|, |b|
 #pragma unroll
         for (int k = 0; k < K; ++k)
         {
@@ -356,9 +383,8 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
             s[k][2] = bi * bi;
             m[0] = max(m[0], mag_bits(r[k]));
             m[1] = max(m[1], mag_bits(bi));
-            if (Mat::checked && i < cnt && a.A.end(lo + i) - a.A.first(lo + i) > kResW) m[2] = mag_bits(1.0);
         }
-        tm.reduce(s, m, [&](const double (&v)[6]) {
+        tm.reduce(s, m, [&](const double (&v)[5]) {
             init = (isnan(v[3]) || isnan(v[4])) ? NAN : (two ? sqrt(v[1]) : v[3]);
             bn = smax(two ? sqrt(v[2]) : (isnan(v[4]) ? 0.0 : v[4]), 1e-300);
             rz = v[0];
@@ -369,16 +395,10 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
                 fin = init;
                 go = false;
             }
-            if (Mat::checked && v[5] > 0.0)
-            {
-                it = -1;  // not this kernel's matrix: x is left as it was
-                go = false;
-            }
             if (threadIdx.x == 0)
             {
                 sc.go = go;
                 sc.beta = 0.0;
-                sc.fits = it >= 0;
             }
         });
     }
@@ -476,7 +496,7 @@ __global__ void __launch_bounds__(kTeamThreads, 1) k_pers_cg(PersCg<Mat> a, Pers
     for (int k = 0; k < K; ++k)
     {
         const int i = threadIdx.x + k * kTeamThreads;
-        if (i < cnt && !tm.dead() && sc.fits) a.x[lo + i] = x[k];
+        if (i < cnt && !tm.dead()) a.x[lo + i] = x[k];
     }
     if (tm.rank == 0 && threadIdx.x == 0)
     {
@@ -807,10 +827,10 @@ void dispatchK(int K, F&& f)
     f(std::integral_constant<int, Kmax>{});
 }
 
-inline TeamMem teamMem(const TeamPlan& tp, int n, unsigned* count, double* part, int* failed)
+inline TeamMem teamMem(const TeamPlan& tp, int n, unsigned* count, double* part, int* failed, long long start = 0)
 {
     return TeamMem{tp.blocks, count, part, (n + kGroupRows - 1) / kGroupRows, tp.chunk / kGroupRows, failed,
-                   teamWaitLimit()};
+                   teamWaitLimit(), start};
 }
 /// doubles of `part` for a system of n rows in one team, and in any plan
 constexpr size_t teamPartMax(int n) { return 2 * kTeamVals * (static_cast<size_t>(n) / kGroupRows + 1); }
@@ -834,13 +854,13 @@ void launchTeam(const TeamPlan& tp, int teams, Kern kernel, const A& args, const
         at[0].val.clusterDim.x = static_cast<unsigned>(tp.blocks);
         at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     }
-    else
+    else if (t.g.start == 0)
     {
         at[0].id = cudaLaunchAttributeCooperative;
         at[0].val.cooperative = 1;
     }
     cfg.attrs = at;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = tp.cluster || t.g.start == 0 ? 1 : 0;
     CFG_CUDA(cudaLaunchKernelEx(&cfg, kernel, args, t));
 }
 

@@ -637,10 +637,12 @@ Ctx::~Ctx()
 
 namespace
 {
-thread_local long long g_teamWait = kTeamWaitCycles;
+thread_local long long g_teamWait = kTeamWaitCycles, g_teamStart = kTeamStartCycles;
 }
 long long teamWaitLimit() { return g_teamWait; }
 void setTeamWaitLimit(long long cycles) { g_teamWait = cycles > 0 ? cycles : kTeamWaitCycles; }
+long long teamStartLimit() { return g_teamStart; }
+void setTeamStartLimit(long long cycles) { g_teamStart = cycles > 0 ? cycles : kTeamStartCycles; }
 
 /// The largest cluster of whole-solve blocks the device runs: 16 (a
 /// non-portable size, which a partitioned GPU may not have), else 8, else 0.

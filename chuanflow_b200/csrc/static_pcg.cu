@@ -31,11 +31,18 @@ namespace
 constexpr int kStaticMaxRows = 1 << 18;  // largest system the static scratch holds
 constexpr int kStaticMaxBlocks = (kStaticMaxRows + RPT * TPB - 1) / (RPT * TPB);
 constexpr size_t kVecBytes = sizeof(double) * kStaticMaxRows;
-constexpr size_t kPartialBytes = sizeof(double) * 16 * kStaticMaxBlocks;
-constexpr size_t kStateBytes = (sizeof(SolveState) + 255) / 256 * 256;
+constexpr size_t kPartialBytes = sizeof(double) * 16 * kStaticMaxBlocks;  // up to 4 values of RPT * kStaticMaxBlocks blocks
+/// the solver state, the resident kernel's failure code, and whether a row of
+/// the matrix is too long for it
+struct StaticState
+{
+    SolveState st;
+    int failed, wide;
+};
+constexpr size_t kStateBytes = (sizeof(StaticState) + 255) / 256 * 256;
 // layout: r, p, Ap, diag (one vector each), block partials, solver state; the
 // resident kernel (persist.cuh) keeps a grid team's partials in r, its gather
-// vector in p and its counters and failure flag in Ap
+// vector in p and its counters in Ap
 static_assert(teamPartMax(kStaticMaxRows) * sizeof(double) <= sizeof(double) * kStaticMaxRows, "partials fit a vector");
 constexpr size_t kScratchBytes = 4 * kVecBytes + kPartialBytes + kStateBytes;
 
@@ -62,19 +69,20 @@ unsigned char* scratchOn(int device)
     return g_scratchAddr[device];
 }
 
-/// Every field of the solver state cleared (tickets, flags, counters), then
-/// the tolerance and iteration limit set: the array keeps the previous
-/// call's contents.
-__global__ void k_static_state_init(SolveState* st, double tol, int maxIter, unsigned* count, int* failed)
+/// Every word of the state cleared (tickets, flags, counters), then the
+/// tolerance and iteration limit set: the array keeps the previous call's
+/// contents.  One block.
+__global__ void k_static_state_init(StaticState* state, double tol, int maxIter, unsigned* count)
 {
-    if (blockIdx.x != 0 || threadIdx.x != 0) return;
-    for (int i = 0; i < kTeamsMax * kCountStride; ++i) count[i] = 0;
-    *failed = 0;
-    unsigned char* b = reinterpret_cast<unsigned char*>(st);
-    for (size_t i = 0; i < sizeof(SolveState); ++i) b[i] = 0;
-    st->tol = tol;
-    st->maxIter = maxIter;
-    st->nComp = 1;
+    static_assert(sizeof(StaticState) % sizeof(unsigned) == 0, "cleared by words");
+    for (int i = threadIdx.x; i < kTeamsMax * kCountStride; i += blockDim.x) count[i] = 0;
+    unsigned* const b = reinterpret_cast<unsigned*>(state);
+    for (int i = threadIdx.x; i < static_cast<int>(sizeof(StaticState) / sizeof(unsigned)); i += blockDim.x) b[i] = 0;
+    __syncthreads();
+    if (threadIdx.x != 0) return;
+    state->st.tol = tol;
+    state->st.maxIter = maxIter;
+    state->st.nComp = 1;
 }
 
 /// One CSR row of A x, columns in the row's order (SparseMatrix::product,
@@ -106,8 +114,9 @@ __global__ void __launch_bounds__(TPB) k_static_cg_init(int n, const int* __rest
                                                         const double* __restrict__ vals, const double* __restrict__ b,
                                                         const double* __restrict__ x, double* __restrict__ r,
                                                         double* __restrict__ p, double* __restrict__ d,
-                                                        double* partials, SolveState* st)
+                                                        double* partials, SolveState* st, const int* wanted)
 {
+    if (wanted && *wanted == 0) return;
     double mx[3] = {0.0, 0.0, 0.0};
     double sm[1] = {0.0};
     FOR_ROWS(c, n)
@@ -229,55 +238,69 @@ extern "C" int cfg_pcg_solve_static(int32_t device, int64_t n64, const int32_t* 
         double* Ap = reinterpret_cast<double*>(base + 2 * kVecBytes);
         double* d = reinterpret_cast<double*>(base + 3 * kVecBytes);
         double* partials = reinterpret_cast<double*>(base + 4 * kVecBytes);
-        SolveState* st = reinterpret_cast<SolveState*>(base + 4 * kVecBytes + kPartialBytes);
+        StaticState* state = reinterpret_cast<StaticState*>(base + 4 * kVecBytes + kPartialBytes);
+        SolveState* st = &state->st;
         cudaStream_t s = static_cast<cudaStream_t>(stream);
         unsigned* count = reinterpret_cast<unsigned*>(Ap);
-        int* failed = reinterpret_cast<int*>(count + kTeamsMax * kCountStride);
-        // one resident kernel while the rows fit (persist.cuh checks their
-        // lengths and leaves x alone when one does not): on a 63^3 system 55 us
-        // an iteration as three launches over uncoalesced CSR rows
-        int sms = 0, coop = 0;
+        // RPT rows per thread; one when it stands in for the resident kernel,
+        // whose order of the sums that is
+        int G = (n + RPT * TPB - 1) / (RPT * TPB);
+        // one resident kernel while the rows fit (persist.cuh measures them
+        // first and leaves x alone when one does not): on a 63^3 system 55 us
+        // an iteration as three launches over uncoalesced CSR rows.  The caller
+        // may keep other work on the GPU, even work that waits for this solve:
+        // a grid takes seven SMs of eight at most (every allowed size fits
+        // them) and no cooperative launch, which would wait for as long as the
+        // other work lasts; when its blocks are not all there in a millisecond
+        // they leave and the per-iteration kernels solve
+        StaticState got{};
+        auto look = [&] {
+            CFG_CUDA(cudaMemcpyAsync(&got, state, sizeof got, cudaMemcpyDeviceToHost, s));
+            CFG_CUDA(cudaStreamSynchronize(s));
+        };
+        auto tell = [&] {
+            const SolveState& h = got.st;
+            report->iterations = h.it[0];
+            report->converged = h.conv[0];
+            report->initial_residual = h.init[0];
+            report->final_residual = (h.conv[0] && h.it[0] == 0) ? h.init[0] : h.fin[0];
+            if (switched) cudaSetDevice(prev);
+            return CFG_OK;
+        };
+        int sms = 0;
         CFG_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device));
-        CFG_CUDA(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, device));
-        if (const TeamPlan tp = teamPlanOf(n, 1, largestCluster(device), sms, coop != 0); tp.blocks)
+        if (const TeamPlan tp = teamPlanOf(n, 1, largestCluster(device), sms - (sms + 7) / 8, true); tp.blocks)
         {
-            k_static_state_init<<<1, 1, 0, s>>>(st, tol, maxIter, count, failed);
+            k_static_state_init<<<1, TPB, 0, s>>>(state, tol, maxIter, count);
             CFG_CUDA(cudaGetLastError());
             using View = CsrView<int>;
             const PersCg<View> a{View{n, rowStart, cols, vals}, b, x, p, nullptr, nullptr, 0};
-            const PersArgs t{tol, maxIter, 0, tp.chunk, st, nullptr, teamMem(tp, n, count, r, failed)};
+            const PersArgs t{tol, maxIter, 0, tp.chunk, st, nullptr,
+                             teamMem(tp, n, count, r, &state->failed, teamStartLimit()), &state->wide};
             dispatchK<kRes1K>(tp.K, [&](auto Kc) {
                 constexpr int K = decltype(Kc)::value;
                 const size_t smem = resident_smem(K, 1, true);
                 if (tp.cluster) launchTeam(tp, 1, k_pers_cg<K, ClusterTeam, false, View>, a, t, smem, s);
                 else launchTeam(tp, 1, k_pers_cg<K, GridTeam, false, View>, a, t, smem, s);
             });
-            SolveState h;
-            int bad = 0;
-            CFG_CUDA(cudaMemcpyAsync(&h, st, sizeof(SolveState), cudaMemcpyDeviceToHost, s));
-            CFG_CUDA(cudaMemcpyAsync(&bad, failed, sizeof(int), cudaMemcpyDeviceToHost, s));
-            CFG_CUDA(cudaStreamSynchronize(s));
-            if (bad) fail(CFG_ECUDA, "cfg_pcg_solve_static: a wait inside a kernel ran out");
-            if (h.it[0] >= 0)
-            {
-                report->iterations = h.it[0];
-                report->converged = h.conv[0];
-                report->initial_residual = h.init[0];
-                report->final_residual = (h.conv[0] && h.it[0] == 0) ? h.init[0] : h.fin[0];
-                if (switched) cudaSetDevice(prev);
-                return CFG_OK;
-            }
+            // a matrix that is too wide for it begins here, without another wait
+            k_static_cg_init<<<G, TPB, 0, s>>>(n, rowStart, cols, vals, b, x, r, p, d, partials, st, &state->wide);
+            CFG_CUDA(cudaGetLastError());
+            look();
+            if (got.failed == kTeamWaitRanOut) fail(CFG_ECUDA, "cfg_pcg_solve_static: a wait inside a kernel ran out");
+            if (got.failed == kTeamNotStarted) G = (n + TPB - 1) / TPB;
+            else if (!got.wide) return tell();
         }
-        const int G = (n + RPT * TPB - 1) / (RPT * TPB);
-        k_static_state_init<<<1, 1, 0, s>>>(st, tol, maxIter, count, failed);
-        k_static_cg_init<<<G, TPB, 0, s>>>(n, rowStart, cols, vals, b, x, r, p, d, partials, st);
-        CFG_CUDA(cudaGetLastError());
-        int allDone = 0;
+        if (!got.wide)
+        {
+            k_static_state_init<<<1, TPB, 0, s>>>(state, tol, maxIter, count);
+            k_static_cg_init<<<G, TPB, 0, s>>>(n, rowStart, cols, vals, b, x, r, p, d, partials, st, nullptr);
+            CFG_CUDA(cudaGetLastError());
+            look();
+        }
         for (int launched = 0, chunk = 8;; chunk = std::min(2 * chunk, 64))
         {
-            CFG_CUDA(cudaMemcpyAsync(&allDone, &st->allDone, sizeof(int), cudaMemcpyDeviceToHost, s));
-            CFG_CUDA(cudaStreamSynchronize(s));
-            if (allDone || launched >= maxIter) break;
+            if (got.st.allDone || launched >= maxIter) return tell();
             const int m = std::min(chunk, maxIter - launched);
             for (int k = 0; k < m; ++k)
             {
@@ -287,16 +310,8 @@ extern "C" int cfg_pcg_solve_static(int32_t device, int64_t n64, const int32_t* 
             }
             CFG_CUDA(cudaGetLastError());
             launched += m;
+            look();
         }
-        SolveState h;
-        CFG_CUDA(cudaMemcpyAsync(&h, st, sizeof(SolveState), cudaMemcpyDeviceToHost, s));
-        CFG_CUDA(cudaStreamSynchronize(s));
-        report->iterations = h.it[0];
-        report->converged = h.conv[0];
-        report->initial_residual = h.init[0];
-        report->final_residual = (h.conv[0] && h.it[0] == 0) ? h.init[0] : h.fin[0];
-        if (switched) cudaSetDevice(prev);
-        return CFG_OK;
     }
     catch (const Error& e)
     {

@@ -53,21 +53,24 @@ __device__ __forceinline__ double mag_value(unsigned long long b)
 
 /// The teams of a launch (one per component of a solve whose components
 /// iterate on their own) and the global-memory side of grid teams: per team
-/// an arrival counter, an exit counter that resets both for the next launch
-/// and two sets of partials; a flag raised when a wait ran out, and the GPU
-/// cycles after which it does.
+/// an arrival counter, an exit counter that resets them for the next launch,
+/// the words of a start that no cooperative launch vouches for, and two sets of
+/// partials; a flag for a wait that ran out (kTeam...), and the GPU cycles after
+/// which it does.
 constexpr int kTeamsMax = 3;
 constexpr int kCountStride = 64;  // a team's counters on lines of their own
 struct TeamMem
 {
     int blocks;        // per team
-    unsigned* count;   // [team][kCountStride]: arrivals at 0, exits at 32
+    unsigned* count;   // [team][kCountStride]: arrivals at 0, exits at 32, a start's arrivals and verdict at 33, 34
     double* part;      // [team][2][kTeamVals][groups]
     int groups;        // 256-row groups of the system
     int perBlock;      // and of one block
     int* failed;
     long long wait;
+    long long start;   // 0: a cooperative launch; else a plain one, whose blocks wait this long for all to be there
 };
+constexpr int kTeamWaitRanOut = 1, kTeamNotStarted = 2;
 
 struct TeamSmem
 {
@@ -290,7 +293,11 @@ struct ClusterTeam
 /// met after `wait` cycles marks the block dead and returns; every body checks
 /// dead() after each sync and reduction, leaves without storing its solution
 /// and still counts itself out, so the counters are ready for the next launch.
+/// A plain launch (`start`) first sees whether every block is there: the last to
+/// arrive says go, a block that has waited too long says no, the first word
+/// counts, and after a no every block leaves before it has written anything.
 constexpr long long kTeamWaitCycles = 4000000000LL;  // about two seconds
+constexpr long long kTeamStartCycles = 2000000LL;    // about a millisecond
 
 /// whether `seen` arrivals have reached `target`, both counted modulo 2^32
 __host__ __device__ constexpr bool arrived(unsigned seen, unsigned target) { return static_cast<int>(seen - target) >= 0; }
@@ -312,8 +319,35 @@ struct GridTeam
           count(g.count + team * kCountStride), part0(g.part + static_cast<size_t>(team) * 2 * kTeamVals * g.groups),
           failed(g.failed), wait(g.wait)
     {
-        if (threadIdx.x == 0) sm.dead = 0;
+        if (threadIdx.x == 0)
+        {
+            sm.dead = 0;
+            if (g.start > 0 && !assembled(g.start))
+            {
+                sm.dead = 1;
+                *static_cast<volatile int*>(failed) = kTeamNotStarted;
+            }
+        }
         __syncthreads();
+    }
+    /// one thread: whether every block of the team is running at once
+    __device__ __forceinline__ bool assembled(long long limit)
+    {
+        unsigned* const verdict = count + kCountStride / 2 + 2;  // 0: open, 1: go, 2: no
+        if (atomicAdd(count + kCountStride / 2 + 1, 1u) == static_cast<unsigned>(nb) - 1u)
+            return atomicCAS(verdict, 0u, 1u) == 0u;
+        const long long t0 = clock64();
+        for (;;)
+        {
+            unsigned seen;
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(verdict) : "memory");
+            if (seen == 0u && clock64() - t0 > limit)
+            {
+                seen = atomicCAS(verdict, 0u, 2u);
+                if (seen == 0u) return false;
+            }
+            if (seen != 0u) return seen == 1u;
+        }
     }
     __device__ __forceinline__ bool dead() const { return sm.dead != 0; }
     /// one thread: arrive (after its own writes) and wait for the others; the
@@ -332,7 +366,7 @@ struct GridTeam
             if (clock64() - t0 > wait)
             {
                 sm.dead = 1;
-                *static_cast<volatile int*>(failed) = 1;
+                *static_cast<volatile int*>(failed) = kTeamWaitRanOut;
                 break;
             }
         }
@@ -381,7 +415,7 @@ struct GridTeam
             if (atomicAdd(count + kCountStride / 2, 1u) == static_cast<unsigned>(nb) - 1u)
             {
                 count[0] = 0;
-                count[kCountStride / 2] = 0;
+                for (int i = 0; i < 3; ++i) count[kCountStride / 2 + i] = 0;
                 __threadfence();
             }
         }

@@ -366,6 +366,10 @@ int cfg_sparse_solve(const cfg_ctx* ctx_or_null, int32_t device, int64_t n, cons
  * fields are then unspecified until they are set again, and its next solve
  * starts clean.  Applies to the solves the calling thread starts from now on. */
 int cfg_solver_wait_limit(int64_t cycles);
+/* GPU clock cycles that cfg_pcg_solve_static's one-kernel form waits for its
+ * blocks to be running at once before the per-iteration kernels take its place
+ * (0 or less: the default, about a millisecond); this thread's solves. */
+int cfg_solver_start_limit(int64_t cycles);
 
 /* ---- the pressure-Poisson solve on its own (no reference counterpart) ---- */
 
@@ -468,8 +472,18 @@ int cfg_gradient(cfg_ctx* ctx, const double* data, const double* bvals, int32_t 
  * this call allocates nothing: its work vectors live in one static device
  * array of the library, sized for at most 262,144 rows (about 8.5 MB, held
  * on every GPU that loads the library until the process exits); larger n is
- * rejected with CFG_EINVAL.  The call waits on its stream once per chunk of
- * iterations to test convergence.  The first call on each device looks that
+ * rejected with CFG_EINVAL.
+ * When no row has more than 7 entries the solve is one kernel, for which the
+ * call waits once: up to 32,768 rows a cluster of at most 16 SMs, which starts
+ * when that many are free; above, one block on each of at most seven SMs of
+ * eight for the length of the solve.  Work on other streams goes on on the
+ * others.  A block waits about a millisecond for the rest to be running too
+ * (cfg_solver_start_limit); when other work holds the SMs for longer, and for
+ * longer rows, the solve runs as kernels per iteration beside that work, and
+ * the call waits on its stream once per chunk of iterations.  The two forms
+ * give the same bits for rows of at most 7 entries.  CFG_ECUDA with a wait
+ * that ran out (cfg_solver_wait_limit): x is unspecified.
+ * The first call on each device looks that
  * array's address up (cudaGetSymbolAddress, with the device current) and
  * keeps it for the life of the process, so make that first call before any
  * stream capture begins; after a cudaDeviceReset on that device the kept

@@ -15,13 +15,36 @@ pytestmark = pytest.mark.gpu
 
 
 @contextlib.contextmanager
-def wait_limit(cycles):
+def limit(name, cycles):
     import chuanflow_b200 as cf
-    assert cf.lib().cfg_solver_wait_limit(C.c_int64(cycles)) == 0
+    assert getattr(cf.lib(), name)(C.c_int64(cycles)) == 0
     try:
         yield
     finally:
-        cf.lib().cfg_solver_wait_limit(C.c_int64(0))
+        getattr(cf.lib(), name)(C.c_int64(0))
+
+
+def wait_limit(cycles):
+    return limit("cfg_solver_wait_limit", cycles)
+
+
+def static_solve(n, width, seed, max_iter=2000):
+    """cfg_pcg_solve_static as a function of nothing: (status, x, report, the exact solution)."""
+    import torch
+    import chuanflow_b200 as cf
+    rs, cols, vals, sol, b = matrix(n, width, np.random.default_rng(seed), True)
+    dev = [torch.from_numpy(a).cuda() for a in (rs.astype(np.int32), cols.astype(np.int32), vals, b)]
+
+    def solve():
+        out = torch.full((n,), 0.25, dtype=torch.float64, device="cuda")
+        rep = cf._capi._Report()
+        torch.cuda.synchronize()
+        rc = cf.lib().cfg_pcg_solve_static(C.c_int32(0), C.c_int64(n), *[C.c_void_p(t.data_ptr()) for t in dev],
+                                           C.c_void_p(out.data_ptr()), C.c_double(1e-12), C.c_int32(max_iter), None,
+                                           C.byref(rep))
+        return rc, out.cpu().numpy(), rep
+
+    return solve, sol
 
 
 @pytest.mark.parametrize("p", ["Jacobi", "DIC"])
@@ -58,3 +81,50 @@ def test_host_csr_leaves_x(method):
         assert solve() == 2 and np.all(x == 3.5)
     assert solve() == 0 and rep.converged
     assert np.linalg.norm(x - sol) < 1e-9 * np.linalg.norm(sol)
+
+
+@pytest.mark.parametrize("n", [32769, 75000, 200000, 262144])
+def test_static_pcg_without_all_its_blocks(n):
+    """Blocks that are not all there in time leave, and the per-iteration
+    kernels give the same bits."""
+    solve, sol = static_solve(n, 7, 5)
+    rc, x, rep = solve()
+    assert rc == 0 and rep.converged and np.linalg.norm(x - sol) < 1e-9 * np.linalg.norm(sol)
+    with limit("cfg_solver_start_limit", 1):
+        rc, y, other = solve()
+    assert rc == 0 and other.iterations == rep.iterations and np.array_equal(x, y)
+    rc, y, _ = solve()
+    assert rc == 0 and np.array_equal(x, y)
+
+
+@pytest.mark.parametrize("n", [32769, 262144])
+def test_static_pcg_wait(n):
+    solve, sol = static_solve(n, 7, 6)
+    with wait_limit(1):
+        assert solve()[0] == 2
+    rc, x, rep = solve()
+    assert rc == 0 and rep.converged and np.linalg.norm(x - sol) < 1e-9 * np.linalg.norm(sol)
+
+
+@pytest.mark.parametrize("n", [2, 300, 513, 32768, 32769, 262144])
+def test_static_pcg_one_long_row(n):
+    """A single row of more than seven entries anywhere sends the whole system
+    to the per-iteration kernels."""
+    import scipy.sparse as sp
+    import torch
+    import chuanflow_b200 as cf
+    for at in {0, n // 2, n - 1}:
+        k = [j for j in range(max(0, at - 6), min(n, at + 7)) if j != at]
+        d = np.full(n, 20.0)
+        w = np.full(len(k), -1.0)
+        A = sp.csr_matrix((np.r_[d, w, w], (np.r_[np.arange(n), np.full(len(k), at), k],
+                                            np.r_[np.arange(n), k, np.full(len(k), at)])), (n, n))
+        sol = np.random.default_rng(at).standard_normal(n)
+        dev = [torch.from_numpy(a).cuda() for a in (A.indptr.astype(np.int32), A.indices.astype(np.int32), A.data, A @ sol)]
+        out = torch.zeros(n, dtype=torch.float64, device="cuda")
+        rep = cf._capi._Report()
+        torch.cuda.synchronize()
+        rc = cf.lib().cfg_pcg_solve_static(C.c_int32(0), C.c_int64(n), *[C.c_void_p(t.data_ptr()) for t in dev],
+                                           C.c_void_p(out.data_ptr()), C.c_double(1e-12), C.c_int32(200), None,
+                                           C.byref(rep))
+        assert rc == 0 and rep.converged and np.linalg.norm(out.cpu().numpy() - sol) < 1e-9 * np.linalg.norm(sol)
