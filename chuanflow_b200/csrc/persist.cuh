@@ -93,12 +93,18 @@ __host__ __device__ constexpr bool resident_regs(int K, int NC, bool jacobiCg) {
 /// per thread do not leave it registers)
 __host__ __device__ constexpr bool resident_xs(int K, int NC) { return NC == 3 && K > 1; }
 
+/// a component's part of the gather vector: its slots, then a slot that holds
+/// zero for the entries a row does not have (a real slot's infinity or NaN
+/// would reach rows that are not coupled to it), padded to 16 bytes
+__host__ __device__ constexpr int resident_stride(int K) { return K * kTeamThreads + 2; }
+
 /// dynamic shared memory of a block holding K * kTeamThreads rows of an
 /// NC-component solve: gather vector, values and column codes, x
 __host__ __device__ constexpr size_t resident_smem(int K, int NC, bool jacobiCg)
 {
-    return static_cast<size_t>(K) * kTeamThreads *
-           (NC * sizeof(double) + (resident_regs(K, NC, jacobiCg) ? 0 : kResW * (sizeof(double) + sizeof(int))) +
+    return static_cast<size_t>(NC) * resident_stride(K) * sizeof(double) +
+           static_cast<size_t>(K) * kTeamThreads *
+           ((resident_regs(K, NC, jacobiCg) ? 0 : kResW * (sizeof(double) + sizeof(int))) +
             (resident_xs(K, NC) ? NC * sizeof(double) : 0));
 }
 
@@ -110,7 +116,7 @@ __host__ __device__ constexpr size_t resident_smem(int K, int NC, bool jacobiCg)
 template <int K, int NC, class Team, bool kRegs>
 struct Resident
 {
-    static constexpr int S = K * kTeamThreads;
+    static constexpr int S = K * kTeamThreads, BS = resident_stride(K);
     static constexpr bool kCluster = Team::kCluster;
     // kRegs: the entries are in registers (one component, few rows per
     // thread), and a row's product reads shared memory for the gathered
@@ -118,7 +124,7 @@ struct Resident
     double rv[kRegs ? K : 1][kResW];
     int rc[kRegs ? K : 1][kResW];
     double* val;  // [kResW][S]
-    double* buf;  // [NC][S]
+    double* buf;  // [NC][BS]
     int* code;    // [kResW][S]
     V3P shared;   // the grid team's copy of buf
     int lo, cnt;
@@ -126,11 +132,12 @@ struct Resident
     __device__ Resident(unsigned char* smem, V3P g, int lo_, int cnt_) : shared(g), lo(lo_), cnt(cnt_)
     {
         buf = reinterpret_cast<double*>(smem);
-        val = buf + NC * S;
+        val = buf + NC * BS;
         code = reinterpret_cast<int*>(val + (kRegs ? 0 : kResW * S));
+        if (threadIdx.x < NC) buf[threadIdx.x * BS + S] = 0.0;
     }
-    /// the block's entries from the SELL rows; slots past the last row and
-    /// past a row's last entry are zero values at slot 0
+    /// the block's entries; slots past the last row and past a row's last entry
+    /// are zero values at the zero slot
     template <class Mat>
     __device__ __forceinline__ void load(const Mat& A, int chunk, int rank)
     {
@@ -150,7 +157,7 @@ struct Resident
             {
                 const long long e = e0 + Mat::step * k;
                 const int col = e < e1 ? A.col(e) : -1;
-                int cd = 0;
+                int cd = S;
                 if (col >= 0)
                 {
                     const int owner = col / chunk, slot = col - owner * chunk;
@@ -181,13 +188,13 @@ struct Resident
     }
     __device__ __forceinline__ double gather(int cd, int q) const
     {
-        if (cd >= 0) return buf[q * S + cd];
+        if (cd >= 0) return buf[q * BS + cd];
         if constexpr (kCluster)
         {
             double v;
             asm volatile("ld.shared::cluster.f64 %0, [%1];"
                          : "=d"(v)
-                         : "r"(static_cast<unsigned>(~cd) + 8u * static_cast<unsigned>(q * S)));
+                         : "r"(static_cast<unsigned>(~cd) + 8u * static_cast<unsigned>(q * BS)));
             return v;
         }
         else return __ldcg(shared.c[q] + ~cd);
@@ -236,7 +243,7 @@ struct Resident
     /// the gather vector's value of slot i, for this block and the others
     __device__ __forceinline__ void put(int i, int q, double v)
     {
-        buf[q * S + i] = v;
+        buf[q * BS + i] = v;
         if constexpr (!kCluster)
             if (i < cnt) shared.c[q][lo + i] = v;
     }
