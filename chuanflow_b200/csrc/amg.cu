@@ -152,10 +152,11 @@ Sweeps jacobi(int m)
 /// one sweep before and after each correction on every level
 Smoother singleSweeps() { return Smoother{jacobi(1), jacobi(1)}; }
 
+constexpr int kSingleSweeps = 2;  // the class whose V-cycle has one sweep on every level
 /// The class of a nonsymmetric operator by theta = max over rows of
 /// sum_j |a_ij - a_ji| / (2 a_ii), a bound of the imaginary parts of D^-1 A:
 /// Chebyshev sweeps amplify eigenvalues far off the real axis.
-int skewOf(double theta) { return theta <= 0.5 ? 0 : (theta <= 0.9 ? 1 : 2); }
+int skewOf(double theta) { return theta <= 0.5 ? 0 : (theta <= 0.9 ? 1 : kSingleSweeps); }
 
 /// One full wave of a grid-stride row kernel of TPB threads: the SMs times
 /// the blocks of this kernel one SM holds at once (its registers decide),
@@ -1425,7 +1426,7 @@ void Ctx::amgValues(AmgUse use, const double* vals, const double* diag, const fl
 /// post-smoothing also forms z.q and beta.
 void Ctx::amgApply(const double* r, double* z)
 {
-    amgCycle(r, z, nullptr, nullptr, true);
+    amgCycle(r, z, nullptr, nullptr, kSingleSweeps);
 }
 
 namespace
@@ -1483,11 +1484,11 @@ Coarse<V> coarseOf(const AmgLevel& L)
 /// Jacobi: theta 0.42 45/25/29/37, 0.71 63/57/49/61, 0.83 87/none/70/87, 0.88
 /// 110/none/90/107): class 1 takes lo 0.3, and only on large levels, where
 /// that is a gain over the launches it adds; class 2 keeps single sweeps.
-Smoother smootherOf(const AmgState& a)
+Smoother smootherOf(const AmgState& a, int skewClass)
 {
     const bool large = a.lv.size() > 1 && a.lv[1].n >= kSellMinRows;
-    if (a.skewClass == 2 || (a.skewClass == 1 && !large)) return singleSweeps();
-    const double lo2 = a.skewClass == 1 ? 0.3 : 0.2, lo4 = a.skewClass == 1 ? 0.3 : 0.1;
+    if (skewClass == kSingleSweeps || (skewClass == 1 && !large)) return singleSweeps();
+    const double lo2 = skewClass == 1 ? 0.3 : 0.2, lo4 = skewClass == 1 ? 0.3 : 0.1;
     return Smoother{large ? chebyshev(4, lo4, 1.9) : chebyshev(2, lo2, 1.9), chebyshev(2, lo2, 1.9)};
 }
 
@@ -1605,7 +1606,7 @@ int coarseKernels(const AmgState& a, const Smoother& sm)
 }
 }  // namespace
 
-void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single, bool swept)
+void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, int skewClass, bool swept)
 {
     if (!amg_) fail(CFG_EINVAL, "amg: the hierarchy is not set up (amgValues)");
     AmgState& a = *amg_;
@@ -1620,19 +1621,18 @@ void Ctx::amgCycle(const double* r, double* z, const double* q, FcgState* st, bo
         launchK(amgPdl(), pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
                 V.dinv, r, V.x, V.r);
     }
-    const Smoother sm = single ? singleSweeps() : smootherOf(a);
-    coarseCycle<float>(a, amgPdl(), sms_, stream_, stop, kScale, sm);
+    coarseCycle<float>(a, amgPdl(), sms_, stream_, stop, kScale, smootherOf(a, skewClass));
     // one block partial per block: the grid is at most G_ blocks, which
     // partials_ holds
     const auto post0 = Wsel == 7 ? k_amg_post0<7> : (Wsel == 16 ? k_amg_post0<16> : k_amg_post0<0>);
     launchK(amgPdl(), post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, stop, A, a.vals32,
             V.dinv, r, V.r, z, q, partials_, st);
-    launchCheck("amg_vcycle", amgCycleKernels(kAmgPressure, single));
+    launchCheck("amg_vcycle", amgCycleKernels(kAmgPressure, skewClass));
 }
 
 /// z_q = V-cycle(b_q) for the three components whose done flag is clear
 /// (the BiCGStab's flags; a converged component keeps its old z_q)
-void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, bool single,
+void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, int skewClass,
                     const std::function<void(int)>& mark)
 {
     if (!amgSlot(use)) fail(CFG_EINVAL, "amg: the hierarchy is not set up (amgValues)");
@@ -1648,20 +1648,17 @@ void Ctx::amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, boo
     launchK(amgPdl(), pre0, waveGrid(reinterpret_cast<const void*>(pre0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32, V.dinv,
             b, x, r);
     if (mark) mark(0);
-    coarseCycle<float4>(a, amgPdl(), sms_, stream_, done, scale, single ? singleSweeps() : smootherOf(a));
+    coarseCycle<float4>(a, amgPdl(), sms_, stream_, done, scale, smootherOf(a, skewClass));
     if (mark) mark(1);
     const auto post0 = Wsel == 7 ? k_amgv_post0<7> : (Wsel == 16 ? k_amgv_post0<16> : k_amgv_post0<0>);
     launchK(amgPdl(), post0, waveGrid(reinterpret_cast<const void*>(post0), sms_, A.n), TPB, 0, stream_, done, A, a.vals32,
             V.dinv, b, r, z);
-    launchCheck("amg_vcycle3", amgCycleKernels(use, single));
+    launchCheck("amg_vcycle3", amgCycleKernels(use, skewClass));
 }
 
-/// what the captured V-cycles of a hierarchy depend on beyond its pointers
-int Ctx::amgVariant(AmgUse use) const
-{
-    const AmgState* a = use == kAmgMomentum ? amgU_.get() : amg_.get();
-    return a ? a->skewClass : 0;
-}
+/// the class of the momentum operator the hierarchy last took its values from
+/// (0 without one), which chooses the sweeps of its V-cycles; the pressure's is 0
+int Ctx::amgSkewClass() const { return amgU_ ? amgU_->skewClass : 0; }
 
 void Ctx::setAmgStrength(double theta)
 {
@@ -1689,10 +1686,10 @@ void Ctx::amgVectors3(AmgUse use)
 }
 
 /// The number of kernels one V-cycle launches.
-int Ctx::amgCycleKernels(AmgUse use, bool single) const
+int Ctx::amgCycleKernels(AmgUse use, int skewClass) const
 {
     const AmgState* a = use == kAmgMomentum ? amgU_.get() : amg_.get();
-    return a ? 2 + coarseKernels(*a, single ? singleSweeps() : smootherOf(*a)) : 0;
+    return a ? 2 + coarseKernels(*a, smootherOf(*a, skewClass)) : 0;
 }
 
 namespace
@@ -1940,7 +1937,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
     else if (Wsel == 16) spmvInit(std::integral_constant<int, 16>{});
     else spmvInit(std::integral_constant<int, 0>{});
     launchCheck("fcgd_init");
-    amgCycle(rr[0], z, nullptr, a.st, false);
+    amgCycle(rr[0], z, nullptr, a.st, 0);
     CFG_CUDA(cudaMemsetAsync(pp[0], 0, static_cast<size_t>(n) * sizeof(double), stream_));
     const auto pick = [&](auto a7, auto a16, auto a0) { return Wsel == 7 ? a7 : (Wsel == 16 ? a16 : a0); };
     const auto spmv = form ? pick(k_fcgd_spmv<7, true>, k_fcgd_spmv<16, true>, k_fcgd_spmv<0, true>)
@@ -1958,7 +1955,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
             launchK(amgPdl(), update, updateGrid, TPB, 0, stream_, A, a.vals32, a.lv[0].dinv, pp[w], q, x, rr[o], rr[w],
                     a.lv[0].x, a.lv[0].r, partials_, a.st);
         else launchK(amgPdl(), k_fcgd_update, GS_, TPB, 0, stream_, n, pp[0], q, x, rr[0], partials_, a.st);
-        amgCycle(rr[w], z, q, a.st, false, form);
+        amgCycle(rr[w], z, q, a.st, 0, form);
         launchCheck("fcgd_iter", form ? 1 : 3);
     };
     for (int launched = 0, chunk = 8;;)
@@ -1987,7 +1984,7 @@ void Ctx::amgFcg(const double* vals, const double* b, double* x, double tol, int
         if (ge) CFG_CUDA(cudaGraphLaunch(ge, stream_));
         else
             for (int k = 0; k < m; ++k) iteration(k);
-        launches_ = counted + static_cast<int64_t>(m) * ((form ? 1 : 3) + amgCycleKernels(kAmgPressure, false));
+        launches_ = counted + static_cast<int64_t>(m) * ((form ? 1 : 3) + amgCycleKernels(kAmgPressure, 0));
         launched += m;
         chunk = std::min(chunk * 2, 32);
     }

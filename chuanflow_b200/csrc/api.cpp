@@ -518,7 +518,7 @@ int cfg_poisson_amg_apply(cfg_ctx* ctx, const double* r, double* z)
 {
     return guard([&] {
         need(ctx && r && z, "cfg_poisson_amg_apply: null argument");
-        ctx->c->poissonAmgApply(r, z);
+        ctx->c->poissonAmgApply(r, z, 2);
     });
 }
 
@@ -526,7 +526,27 @@ int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32
 {
     return guard([&] {
         need(ctx && r && z && done, "cfg_poisson_amg_apply3: null argument");
-        ctx->c->poissonAmgApply3(r, z, done);
+        ctx->c->poissonAmgApply3(r, z, done, 2);
+    });
+}
+
+int cfg_poisson_amg_cycle(cfg_ctx* ctx, const double* r, double* z, int32_t vectors, int32_t skewClass)
+{
+    return guard([&] {
+        need(ctx && r && z, "cfg_poisson_amg_cycle: null argument");
+        need(vectors == 1 || vectors == 3, "cfg_poisson_amg_cycle: one vector or three");
+        need(skewClass >= 0 && skewClass <= 2, "cfg_poisson_amg_cycle: class out of range");
+        const int32_t done[3] = {0, 0, 0};
+        if (vectors == 1) ctx->c->poissonAmgApply(r, z, skewClass);
+        else ctx->c->poissonAmgApply3(r, z, done, skewClass);
+    });
+}
+
+int cfg_amg_momentum_class(const cfg_ctx* ctx, int32_t* skewClass)
+{
+    return guard([&] {
+        need(ctx && skewClass, "cfg_amg_momentum_class: null argument");
+        *skewClass = ctx->c->amgSkewClass();
     });
 }
 

@@ -269,8 +269,9 @@ public:
                       double innerTol, double* out);
     /// the AMG hierarchy for the Poisson system's current values
     void poissonAmg(double* out);
-    void poissonAmgApply(const double* r, double* z);
-    void poissonAmgApply3(const double* r, double* z, const int32_t done[3]);
+    void poissonAmgApply(const double* r, double* z, int skewClass);
+    void poissonAmgApply3(const double* r, double* z, const int32_t done[3], int skewClass);
+    int amgSkewClass() const;
     /// strength threshold of the pressure hierarchy's aggregation (0: plain);
     /// fixed once that hierarchy is built
     void setAmgStrength(double theta);
@@ -305,18 +306,17 @@ private:
     void amgSetup(AmgUse use, const double* vals, double theta);
     void amgValues(AmgUse use, const double* vals, const double* diag, const float* vals32);
     void amgApply(const double* r, double* z);
-    /// single: one sweep before and after each correction on every level, else
-    /// the hierarchy's own smoothers on the coarse ones; swept: the finest
-    /// first sweep and residual are there already
-    void amgCycle(const double* r, double* z, const double* q, FcgState* st, bool single,
+    /// skewClass: of the operator, which chooses the sweeps of the coarse
+    /// levels (smootherOf; 2: one sweep everywhere); swept: the finest first
+    /// sweep and residual are there already
+    void amgCycle(const double* r, double* z, const double* q, FcgState* st, int skewClass,
                   bool swept = false);
     /// mark(0) after the finest pre-sweep, mark(1) before the finest
     /// post-sweep (kernel timing), when given
-    void amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, bool single,
+    void amgCycle3(AmgUse use, CV3P b, V3P z, const int* done, float scale, int skewClass,
                    const std::function<void(int)>& mark = {});
     void amgVectors3(AmgUse use);
-    int amgCycleKernels(AmgUse use, bool single) const;
-    int amgVariant(AmgUse use) const;
+    int amgCycleKernels(AmgUse use, int skewClass) const;
     void amgFcg(const double* vals, const double* b, double* x, double tol, int maxIter, int normType,
                 cfg_solver_report* rep);
     void amgInfo(double* out);

@@ -1789,7 +1789,7 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
     init.nComp = 3;
     const int n = dm_.nC;
     const int* done = reinterpret_cast<const int*>(reinterpret_cast<const char*>(st_) + offsetof(SolveState, done));
-    const int vk = amgCycleKernels(kAmgMomentum, false);
+    const int skewClass = amgSkewClass(), vk = amgCycleKernels(kAmgMomentum, skewClass);
     CFG_CUDA(cudaMemcpyAsync(st_, &init, sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     auto loop = [&](auto Wc) {
         constexpr int W = decltype(Wc)::value;
@@ -1817,20 +1817,20 @@ void Ctx::runBiCGAmg(const double* vals, const double* diag, V3P b, V3P x, doubl
             for (int q = 0; q < 3; ++q) activeBefore += stHost_->done[q] ? 0 : 1;
             if (stHost_->allDone || launched >= maxIter) break;
             const int m = ktime_ ? 1 : std::min(chunk, maxIter - launched);
-            launchChunk(ptrKey("bicga", {vals, diag, x.c[0], x.c[1], x.c[2]}, W * 4 + amgVariant(kAmgMomentum)), m, [&](int k) {
+            launchChunk(ptrKey("bicga", {vals, diag, x.c[0], x.c[1], x.c[2]}, W * 4 + skewClass), m, [&](int k) {
                 const std::function<void(int)> markZ = [&](int j) { tmark(k, 2 + j); };
                 const std::function<void(int)> markS = [&](int j) { tmark(k, 7 + j); };
                 tmark(k, 0);
                 launchK(amgPdl(), k_bia_p<3>, GS_, TPB, 0, stream_, n, br_, bp_, bv_, st_);
                 tmark(k, 1);
-                amgCycle3(kAmgMomentum, cv(bp_), bz_, done, kAmgScaleMomentum, false,
+                amgCycle3(kAmgMomentum, cv(bp_), bz_, done, kAmgScaleMomentum, skewClass,
                           ktime_ ? markZ : std::function<void(int)>{});
                 tmark(k, 4);
                 launchK(amgPdl(), k_bi_spmv1<W, 3>, GS_, TPB, 0, stream_, A, vals, bz_, bv_, br0_, partials_, st_);
                 tmark(k, 5);
                 launchK(amgPdl(), k_bia_s<3>, GS_, TPB, 0, stream_, n, br_, bv_, bs_, st_);
                 tmark(k, 6);
-                amgCycle3(kAmgMomentum, cv(bs_), bsh_, done, kAmgScaleMomentum, false,
+                amgCycle3(kAmgMomentum, cv(bs_), bsh_, done, kAmgScaleMomentum, skewClass,
                           ktime_ ? markS : std::function<void(int)>{});
                 tmark(k, 9);
                 launchK(amgPdl(), k_bia_spmv2<W, 3>, GS_, TPB, 0, stream_, A, vals, bsh_, bs_, bt_, partials_, st_);
@@ -2956,7 +2956,7 @@ void Ctx::poissonAmg(double* out)
     amgInfo(out);
 }
 
-void Ctx::poissonAmgApply(const double* r, double* z)
+void Ctx::poissonAmgApply(const double* r, double* z, int skewClass)
 {
     if (!amgFresh_)
     {
@@ -2964,11 +2964,11 @@ void Ctx::poissonAmgApply(const double* r, double* z)
         poissonAmg(info);
     }
     toDevCells(cr_, r, 1, 0);
-    amgApply(cr_, cz_);
+    amgCycle(cr_, cz_, nullptr, nullptr, skewClass);
     fromDevCells(z, cz_, 1, 0);
 }
 
-void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3])
+void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3], int skewClass)
 {
     if (!amgFresh_)
     {
@@ -2986,7 +2986,7 @@ void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3])
     // the pressure V-cycle's coarse-correction scale, so that each component
     // equals the single V-cycle's result
     amgCycle3(kAmgPressure, cv(bp_), bz_, reinterpret_cast<const int*>(reinterpret_cast<const char*>(st_) + offsetof(SolveState, done)),
-              kAmgScalePressure, true);
+              kAmgScalePressure, skewClass);
     for (int q = 0; q < 3; ++q) fromDevCells(z + static_cast<size_t>(q) * dm_.nC, bz_.c[q], 1, 0);
 }
 

@@ -426,6 +426,16 @@ int cfg_poisson_amg_apply(cfg_ctx* ctx, const double* r, double* z);
  * values); component q is skipped, its z left as given, when done[q] != 0.
  * Each applied component equals cfg_poisson_amg_apply of it, for tests. */
 int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32_t done[3]);
+/* The V-cycle as the solvers apply it to one vector or to three (3 n values),
+ * for tests: the sweeps of the coarse levels as for an operator of skew_class 0
+ * (CFG_POISSON_FCG_AMG and the AMG pressure solves: near symmetric), 1 or 2 (one
+ * sweep everywhere: the two calls above, and the V-cycle of
+ * CFG_POISSON_FCG_AMG_MPNN).  By theta = max over rows of
+ * sum_j |a_ij - a_ji| / (2 a_ii): 0 up to 0.5, 1 up to 0.9, else 2. */
+int cfg_poisson_amg_cycle(cfg_ctx* ctx, const double* r, double* z, int32_t vectors, int32_t skew_class);
+/* The class of the momentum matrix that the last AMG momentum solve took its
+ * hierarchy's values from (0 before the first), for tests. */
+int cfg_amg_momentum_class(const cfg_ctx* ctx, int32_t* skew_class);
 /* Strength-of-connection aggregation for the pressure AMG hierarchy (the one
  * the SIMPLE and PISO pressure solves and the Poisson system use; no
  * counterpart in the reference, whose pressure solve is Jacobi-PCG,
