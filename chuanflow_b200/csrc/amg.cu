@@ -299,7 +299,8 @@ __global__ void __launch_bounds__(TPB) k_amg_galerkin(int nnz, const int* __rest
     }
 }
 
-/// max over rows of sum_j |a_ij - a_ji| / (2 a_ii), into the bits of *out
+/// max over rows of sum_j |a_ij - a_ji| / (2 a_ii), into the bits of *out; a
+/// row with a NaN counts as 1e300
 __global__ void __launch_bounds__(TPB) k_amg_skew(DMat A, const double* __restrict__ val, unsigned long long* out)
 {
     double mx[1] = {0.0};
@@ -332,10 +333,8 @@ __global__ void __launch_bounds__(TPB) k_amg_skew(DMat A, const double* __restri
             s += fabs(v - w);
         }
         const double t = d > 0.0 ? s / (2.0 * d) : 1.0;
-        if (!(t <= mx[0])) mx[0] = t;  // a NaN stays
+        mx[0] = smax(mx[0], isnan(t) ? 1e300 : t);  // a NaN counts as the worst
     }
-    // NaN counts as the worst
-    if (isnan(mx[0])) mx[0] = 1e300;
     block_max<1>(mx);
     if (threadIdx.x == 0) atomicMax(out, static_cast<unsigned long long>(__double_as_longlong(mx[0])));
 }
