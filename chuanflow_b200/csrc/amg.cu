@@ -1295,7 +1295,7 @@ void Ctx::amgSetup(AmgUse use, const double* vals, double theta)
         for (int k = 0; k < kTailBlocks; ++k)
             nnz = std::max(nnz, rs[static_cast<size_t>(tailFirst(n, k + 1))] - rs[static_cast<size_t>(tailFirst(n, k))]);
         const int nc = a->lv[static_cast<size_t>(T) + 1].n, all = rs[static_cast<size_t>(n)];
-        a->tailCluster = all > kTailClusterEntries;
+        a->tailCluster = all > kTailClusterEntries && clusterMax_ >= kTailBlocks;
         if (!a->tailCluster) nnz = all;
         const size_t bytes = 4 * (a->tailCluster ? tailSmemWords(n, nnz, nc) : tailBlockWords(n, nnz, nc));
         int optin = 0;

@@ -1477,9 +1477,9 @@ std::string ptrKey(const char* kind, std::initializer_list<const void*> ps, int 
 /// thread = 32,768 rows (1,320 rows 31 -> 7.9 ms, 16,000 rows 146 -> 39 ms,
 /// 22,743 rows with k-epsilon 43 -> 17 ms; a grid there took 20, 71 and 21
 /// ms, its barriers costing six of a cluster's); then a grid per component
-/// while the rows fit (62,720 rows 70 -> 37 ms, 102,400 rows 93 -> 52 ms),
-/// then one grid for the three together (131,072 rows 100 -> 53 ms, with DIC
-/// 89 -> 54 ms).  Larger systems stream from memory anyway and keep the
+/// while the rows fit, 100,352 on 148 SMs (62,720 rows 70 -> 37 ms), then one
+/// grid for the three together (102,400 rows 93 -> 52 ms, 131,072 rows 100 ->
+/// 53 ms, with DIC 89 -> 54 ms).  Larger systems stream from memory anyway and keep the
 /// per-iteration kernels.  Detail blocks and captured passes run side by
 /// side with others on the device and never take a grid, which wants every
 /// SM at once: their clusters do not depend on the schedule.
@@ -1506,7 +1506,7 @@ TeamPlan teamPlanOf(int n, int nComp, int clusterMax, int sms, bool gridOk)
     }
     if (tp.blocks)
     {
-        tp.K = perThread(tp.blocks);
+        tp.K = tp.NC == 3 ? kRes3K : perThread(tp.blocks);
         tp.chunk = perBlock(tp.blocks) * kGroupRows;
     }
     return tp;
@@ -1537,10 +1537,8 @@ void Ctx::teamBi(const TeamPlan& tp, int nComp, const double* vals, const double
 {
     const PersBi<SellView> a{{DMat{dm_.nC, dm_.mStart, dm_.mCol}, vals, diag}, b, x, bz_};
     if (tp.NC == 3)
-        dispatchK<kRes3K>(tp.K, [&](auto Kc) {
-            constexpr int K = decltype(Kc)::value;
-            teamLaunch(tp, 1, k_pers_bicg<K, GridTeam, 3, SellView>, a, resident_smem(K, 3, false), tol, maxIter, 0);
-        });
+        // two rows per thread: fewer rows fit a grid per component
+        teamLaunch(tp, 1, k_pers_bicg<kRes3K, GridTeam, 3, SellView>, a, resident_smem(kRes3K, 3, false), tol, maxIter, 0);
     else
         dispatchK<kRes1K>(tp.K, [&](auto Kc) {
             constexpr int K = decltype(Kc)::value;
