@@ -555,6 +555,11 @@ int cfg_solver_wait_limit(int64_t cycles)
     return guard([&] { cfg::setTeamWaitLimit(cycles); });
 }
 
+int cfg_solver_grid_solves(int32_t solves)
+{
+    return guard([&] { cfg::setGridSolvesLimit(solves); });
+}
+
 int cfg_solver_start_limit(int64_t cycles)
 {
     return guard([&] { cfg::setTeamStartLimit(cycles); });

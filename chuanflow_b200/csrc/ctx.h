@@ -25,6 +25,8 @@ struct TeamPlan
     bool cluster = false;
     int NC = 1;      // components per team
     int K = 0, chunk = 0;
+    bool shared = false;  // a grid would have solved, but the device has other solves: the
+                          // per-iteration kernels, one row per thread, give its bits
 };
 TeamPlan teamPlanOf(int n, int nComp, int clusterMax, int sms, bool gridOk);
 int largestCluster(int device);
@@ -35,6 +37,23 @@ void setTeamWaitLimit(long long cycles);
 /// and those that the blocks of a plain launch wait for all to be there
 /// (cfg_solver_start_limit)
 long long teamStartLimit();
+/// the solves at once on a device up to which one of them still takes a grid
+/// team (cfg_solver_grid_solves)
+int gridSolvesLimit();
+void setGridSolvesLimit(int solves);
+/// A solve of a context, or a pass of a batch of them, in progress on a device.
+class SolveScope
+{
+public:
+    explicit SolveScope(int device);
+    ~SolveScope();
+    SolveScope(const SolveScope&) = delete;
+    SolveScope& operator=(const SolveScope&) = delete;
+    static int running(int device);
+
+private:
+    int device_;
+};
 void setTeamStartLimit(long long cycles);
 
 struct Timing
@@ -95,6 +114,7 @@ public:
     /// polling, for enqueueOuter under stream capture.
     void setDeviceLoops(bool on) { devLoop_ = on; }
     cudaStream_t stream() const { return stream_; }
+    int device() const { return device_; }
     /// the inner iteration counts a device-loop iteration left in the
     /// scalars: momentum, pressure, RANS model
     void deviceInner(int64_t& u, int64_t& p, int64_t& t) const;
@@ -255,7 +275,7 @@ private:
     template <class T>
     void dicSetupT(DDicT<T>& D, const double* vals, const T* diag);
     template <class T>
-    void dicApplyT(const DDicT<T>& D, const T* r, T* z);
+    void dicApplyT(const DDicT<T>& D, const T* r, T* z, bool rowSums = false);
     template <class T>
     void dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T* x, T* r, T* p, T* Ap, T* z, double tol,
                 int maxIter, int normType, cfg_solver_report* rep);
@@ -367,6 +387,7 @@ private:
     bool savedTurb_ = false;
     void turbCopy(double* buf, bool save);
     int rowGrid(int rows) const;
+    int solverGrid(const TeamPlan& tp) const { return tp.shared ? (dm_.nC + TPB - 1) / TPB : GS_; }
     int maxW_ = 0;     // longest matrix row
     int nSlicesEntries_ = 0;  // matrix SELL entries
     int nSlices_ = 0;

@@ -537,6 +537,8 @@ void batchPassGraph(cfg_batch& b, const double* q, const cfg_simple_controls* ct
                     double* wallMs)
 {
     const int n = static_cast<int>(b.blocks.size());
+    std::unique_ptr<SolveScope> scope;
+    if (n > 0) scope = std::make_unique<SolveScope>(b.blocks[0]->device());
     for (cfg::Ctx* c : b.blocks)
         c->setRowBlocks(b.rowBlocks >= 0 ? b.rowBlocks
                                          : static_cast<int>(std::min<int64_t>(4, std::max<int64_t>(

@@ -182,6 +182,27 @@ __global__ void __launch_bounds__(TPB, kSolverMinBlocks) k_dic_bwd(DDicT<T> D, D
     }
 }
 
+/// r.z in the order of the rows, and beta (as the last phase of k_dic_bwd)
+template <class T>
+__global__ void __launch_bounds__(TPB, kSolverMinBlocks) k_dic_rz(int n, const T* __restrict__ r, const T* __restrict__ z,
+                                                                  double* partials, SolveState* st)
+{
+    if (st->allDone) return;
+    double sm[1] = {0.0};
+    FOR_ROWS(c, n) sm[0] += static_cast<double>(r[c] * z[c]);
+    block_sum<1>(sm);
+    if (threadIdx.x == 0) partials[blockIdx.x] = sm[0];
+    if (!last_block(&st->ticket[0])) return;
+    double fs[1];
+    final_sum<1>(partials, gridDim.x, fs);
+    if (threadIdx.x == 0)
+    {
+        st->ticket[0] = 0;
+        st->beta[0] = st->it[0] == 0 ? 0.0 : fs[0] / st->rz[0];
+        st->rz[0] = fs[0];
+    }
+}
+
 /// x += alpha p; r -= alpha Ap; residual test (Matrix.cpp:195-208), without z
 template <class T = double>
 __global__ void __launch_bounds__(TPB, kSolverMinBlocks) k_cg_update_nz(int n, const T* __restrict__ p, const T* __restrict__ Ap,

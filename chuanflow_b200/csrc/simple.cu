@@ -1,6 +1,7 @@
 // The SIMPLE outer iteration on the device (src/3d/src/solvers/simpleSolver.cpp:33-394)
 // and the host driver that sequences its kernels.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -643,6 +644,25 @@ long long teamWaitLimit() { return g_teamWait; }
 void setTeamWaitLimit(long long cycles) { g_teamWait = cycles > 0 ? cycles : kTeamWaitCycles; }
 long long teamStartLimit() { return g_teamStart; }
 void setTeamStartLimit(long long cycles) { g_teamStart = cycles > 0 ? cycles : kTeamStartCycles; }
+
+namespace
+{
+// More solves than this at once on a device and no context's takes a grid, which
+// holds every SM for the length of a solve: they would take turns.  Jacobi
+// channels on several threads, ms per solve of each, always a grid / with this
+// rule / per-iteration kernels only: four of 62,720 rows 86 / 54 / 54, eight of
+// 35,280 rows 160 / 59 / 59, one of 16,000 rows (a cluster) and one of 62,720
+// 25 and 25 / 8.6 and 46 / 8.5 and 46; a context of 62,720 rows alone 23 / 23 / 45.
+constexpr int kGridSolves = 1;
+thread_local int g_gridSolves = kGridSolves;
+constexpr int kScopes = 64;
+std::atomic<int> g_running[kScopes];
+}
+int gridSolvesLimit() { return g_gridSolves; }
+void setGridSolvesLimit(int solves) { g_gridSolves = solves < 0 ? kGridSolves : solves; }
+SolveScope::SolveScope(int device) : device_(device % kScopes) { ++g_running[device_]; }
+SolveScope::~SolveScope() { --g_running[device_]; }
+int SolveScope::running(int device) { return g_running[device % kScopes]; }
 
 /// The largest cluster of whole-solve blocks the device runs: 16 (a
 /// non-portable size, which a partitioned GPU may not have), else 8, else 0.
@@ -1519,7 +1539,13 @@ TeamPlan Ctx::teamPlan(int nComp, bool bicg) const
     // the per-iteration kernels, which have one row per thread up to initGS_
     // blocks
     if (ktime_ || maxW_ > kResW || (bicg && nComp == 1 && dm_.nC > initGS_ * TPB)) return TeamPlan{};
-    return teamPlanOf(dm_.nC, nComp, clusterMax_, sms_, coopOk_ && !detail_ && !devLoop_);
+    TeamPlan tp = teamPlanOf(dm_.nC, nComp, clusterMax_, sms_, coopOk_ && !detail_ && !devLoop_);
+    if (tp.blocks && !tp.cluster && SolveScope::running(device_) > gridSolvesLimit())
+    {
+        tp = TeamPlan{};
+        tp.shared = true;
+    }
+    return tp;
 }
 
 /// Launches a whole-solve kernel as its team.
@@ -1592,7 +1618,9 @@ void Ctx::runCG(const double* vals, const double* diag, const double* b, double*
                 cfg_solver_report* rep, int normType)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
-    if (const TeamPlan tp = teamPlan(1, false); tp.blocks)
+    const TeamPlan tp = teamPlan(1, false);
+    const int G = solverGrid(tp);
+    if (tp.blocks)
     {
         teamCg<false>(tp, vals, diag, b, x, nullptr, tol, maxIter, normType);
         teamReport(1, rep);
@@ -1628,7 +1656,7 @@ void Ctx::runCG(const double* vals, const double* diag, const double* b, double*
     }
     dispatchW(maxW_, [&](auto Wc) {
         constexpr int W = decltype(Wc)::value;
-        k_cg_init<W><<<GS_, TPB, 0, stream_>>>(A, vals, diag, b, x, cr_, cp_, partials_, st_);
+        k_cg_init<W><<<G, TPB, 0, stream_>>>(A, vals, diag, b, x, cr_, cp_, partials_, st_);
         launchCheck("cg_init");
         int launched = 0;
         int chunk = 8;
@@ -1646,13 +1674,13 @@ void Ctx::runCG(const double* vals, const double* diag, const double* b, double*
             itBefore = stHost_->it[0];
             if (stHost_->allDone || launched >= maxIter) break;
             const int n = std::min(chunk, maxIter - launched);
-            launchChunk(ptrKey("cg", {vals, diag, x}, W), n, [&](int k) {
+            launchChunk(ptrKey("cg", {vals, diag, x}, W * 2 + tp.shared), n, [&](int k) {
                 tmark(k, 0);
-                k_cg_spmv<W><<<GS_, TPB, 0, stream_>>>(A, vals, cp_, cAp_, partials_, st_);
+                k_cg_spmv<W><<<G, TPB, 0, stream_>>>(A, vals, cp_, cAp_, partials_, st_);
                 tmark(k, 1);
-                k_cg_update<double><<<GS_, TPB, 0, stream_>>>(dm_.nC, diag, cp_, cAp_, x, cr_, partials_, st_);
+                k_cg_update<double><<<G, TPB, 0, stream_>>>(dm_.nC, diag, cp_, cAp_, x, cr_, partials_, st_);
                 tmark(k, 2);
-                k_cg_p<double><<<GS_, TPB, 0, stream_>>>(dm_.nC, diag, cr_, cp_, st_);
+                k_cg_p<double><<<G, TPB, 0, stream_>>>(dm_.nC, diag, cr_, cp_, st_);
                 tmark(k, 3);
                 launchCheck("cg_iter", 0);
             });
@@ -1672,7 +1700,9 @@ void Ctx::runBiCG3(const double* vals, const double* diag, V3P b, V3P x, int nCo
                    cfg_solver_report* reps)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
-    if (const TeamPlan tp = teamPlan(nComp, true); tp.blocks)
+    const TeamPlan tp = teamPlan(nComp, true);
+    const int G = solverGrid(tp);
+    if (tp.blocks)
     {
         teamBi(tp, nComp, vals, diag, b, x, tol, maxIter);
         teamReport(nComp, reps);
@@ -1715,7 +1745,7 @@ void Ctx::runBiCG3(const double* vals, const double* diag, V3P b, V3P x, int nCo
     auto loop = [&](auto Wc, auto NCc) {
         constexpr int W = decltype(Wc)::value;
         constexpr int NC = decltype(NCc)::value;
-        k_bi_init<W, NC><<<GS_, TPB, 0, stream_>>>(A, vals, diag, bInvD_, b, x, br_, br0_, bp_, bv_, partials_, st_);
+        k_bi_init<W, NC><<<G, TPB, 0, stream_>>>(A, vals, diag, bInvD_, b, x, br_, br0_, bp_, bv_, partials_, st_);
         launchCheck("bicg_init");
         int itBefore = 0, lastChunk = 0, activeBefore = NC;
         auto itMax = [&] {
@@ -1739,15 +1769,15 @@ void Ctx::runBiCG3(const double* vals, const double* diag, V3P b, V3P x, int nCo
             // timed launches go one iteration at a time, so each is charged
             // with the components that were still iterating
             const int m = ktime_ ? 1 : std::min(chunk, maxIter - launched);
-            launchChunk(ptrKey("bicg", {vals, diag, x.c[0], x.c[1], x.c[2]}, W * 8 + NC), m, [&](int k) {
+            launchChunk(ptrKey("bicg", {vals, diag, x.c[0], x.c[1], x.c[2]}, (W * 8 + NC) * 2 + tp.shared), m, [&](int k) {
                 tmark(k, 0);
-                k_bi_p<NC><<<GS_, TPB, 0, stream_>>>(n, bInvD_, br_, bp_, bv_, bz_, st_);
+                k_bi_p<NC><<<G, TPB, 0, stream_>>>(n, bInvD_, br_, bp_, bv_, bz_, st_);
                 tmark(k, 1);
-                k_bi_spmv1<W, NC><<<GS_, TPB, 0, stream_>>>(A, vals, bz_, bv_, br0_, partials_, st_);
+                k_bi_spmv1<W, NC><<<G, TPB, 0, stream_>>>(A, vals, bz_, bv_, br0_, partials_, st_);
                 tmark(k, 2);
-                k_bi_spmv2<W, NC><<<GS_, TPB, 0, stream_>>>(A, vals, bInvD_, br_, bv_, bt_, partials_, st_);
+                k_bi_spmv2<W, NC><<<G, TPB, 0, stream_>>>(A, vals, bInvD_, br_, bv_, bt_, partials_, st_);
                 tmark(k, 3);
-                k_bi_x<NC><<<GS_, TPB, 0, stream_>>>(n, bInvD_, x, bz_, bv_, bt_, br_, br0_, partials_, st_);
+                k_bi_x<NC><<<G, TPB, 0, stream_>>>(n, bInvD_, x, bz_, bv_, bt_, br_, br0_, partials_, st_);
                 tmark(k, 4);
                 launchCheck("bicg_iter", 0);
             });
@@ -1877,8 +1907,16 @@ void Ctx::dicSetupT(DDicT<T>& D, const double* vals, const T* diag)
     });
 }
 
+namespace
+{
+/// the kernels of one application of a DIC of C colours
+int dicKernels(int C, bool rowSums) { return 2 * C - 1 + (C == 1 || rowSums ? 1 : 0); }
+}  // namespace
+
+/// z = M^-1 r and the solver's r.z and beta.  rowSums: r.z in the order of the
+/// rows (the resident solve's), in a kernel of its own, not by colours.
 template <class T>
-void Ctx::dicApplyT(const DDicT<T>& D, const T* r, T* z)
+void Ctx::dicApplyT(const DDicT<T>& D, const T* r, T* z, bool rowSums)
 {
     const int C = D.nColours;
     dispatchW(maxW_, [&](auto Wc) {
@@ -1886,7 +1924,7 @@ void Ctx::dicApplyT(const DDicT<T>& D, const T* r, T* z)
         for (int c = 0; c < C; ++c)
             k_dic_fwd<W, T><<<rowGrid(dicPhase_[c].cnt), TPB, 0, stream_>>>(D, dicPhase_[c], r, z, c == C - 1,
                                                                             partials_, st_);
-        if (C == 1)
+        if (C == 1 && !rowSums)
         {
             // no backward phase: a one-block final reduction of the forward partials
             const DicPhase none{0, 0, 0, dicPartials_ - 1};
@@ -1894,9 +1932,10 @@ void Ctx::dicApplyT(const DDicT<T>& D, const T* r, T* z)
         }
         for (int c = C - 2; c >= 0; --c)
             k_dic_bwd<W, T><<<rowGrid(dicPhase_[c].cnt), TPB, 0, stream_>>>(
-                D, dicPhase_[c], r, z, c == 0, c == 0 ? dicPartials_ - 1 : 0, partials_, st_);
+                D, dicPhase_[c], r, z, c == 0 && !rowSums, c == 0 ? dicPartials_ - 1 : 0, partials_, st_);
+        if (rowSums) k_dic_rz<T><<<(dm_.nC + TPB - 1) / TPB, TPB, 0, stream_>>>(dm_.nC, r, z, partials_, st_);
     });
-    launchCheck("dic_apply", C == 1 ? 2 : 2 * C - 1);
+    launchCheck("dic_apply", dicKernels(C, rowSums));
 }
 
 void Ctx::dicSetup(const double* vals, const double* diag) { dicSetupT<double>(dic_, vals, diag); }
@@ -1909,15 +1948,18 @@ void Ctx::dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T*
                  double tol, int maxIter, int normType, cfg_solver_report* rep)
 {
     const DMat A{dm_.nC, dm_.mStart, dm_.mCol};
+    TeamPlan tp;
     if constexpr (std::is_same<T, double>::value)
     {
-        if (const TeamPlan tp = teamPlan(1, false); tp.blocks)
+        tp = teamPlan(1, false);
+        if (tp.blocks)
         {
             teamCg<true>(tp, vals, diag, b, x, D.rDinv, tol, maxIter, normType);
             teamReport(1, rep);
             return;
         }
     }
+    const int G = solverGrid(tp);
     SolveState init{};
     init.tol = tol;
     init.maxIter = maxIter;
@@ -1951,10 +1993,10 @@ void Ctx::dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T*
     CFG_CUDA(cudaMemcpyAsync(st_, &init, sizeof(SolveState), cudaMemcpyHostToDevice, stream_));
     dispatchW(maxW_, [&](auto Wc) {
         constexpr int W = decltype(Wc)::value;
-        k_cg_init<W, T><<<GS_, TPB, 0, stream_>>>(A, vals, diag, b, x, r, p, partials_, st_);
+        k_cg_init<W, T><<<G, TPB, 0, stream_>>>(A, vals, diag, b, x, r, p, partials_, st_);
         launchCheck("cg_init");
-        dicApplyT<T>(D, r, z);
-        k_cg_pz<T><<<GS_, TPB, 0, stream_>>>(dm_.nC, z, p, st_);
+        dicApplyT<T>(D, r, z, tp.shared);
+        k_cg_pz<T><<<G, TPB, 0, stream_>>>(dm_.nC, z, p, st_);
         launchCheck("cg_pz");
         int launched = 0;
         int chunk = 8;
@@ -1972,19 +2014,19 @@ void Ctx::dicCGT(const DDicT<T>& D, const T* vals, const T* diag, const T* b, T*
             if (stHost_->allDone || launched >= maxIter) break;
             const int n = std::min(chunk, maxIter - launched);
             lastChunk = n;
-            launchChunk(ptrKey("diccg", {vals, diag, x, r, p, Ap, z, D.lVal}, W), n, [&](int k) {
+            launchChunk(ptrKey("diccg", {vals, diag, x, r, p, Ap, z, D.lVal}, W * 2 + tp.shared), n, [&](int k) {
                 tmark(k, 0);
-                k_cg_spmv<W, T><<<GS_, TPB, 0, stream_>>>(A, vals, p, Ap, partials_, st_);
+                k_cg_spmv<W, T><<<G, TPB, 0, stream_>>>(A, vals, p, Ap, partials_, st_);
                 tmark(k, 1);
-                k_cg_update_nz<T><<<GS_, TPB, 0, stream_>>>(dm_.nC, p, Ap, x, r, partials_, st_);
+                k_cg_update_nz<T><<<G, TPB, 0, stream_>>>(dm_.nC, p, Ap, x, r, partials_, st_);
                 tmark(k, 2);
-                dicApplyT<T>(D, r, z);
+                dicApplyT<T>(D, r, z, tp.shared);
                 tmark(k, 3);
-                k_cg_pz<T><<<GS_, TPB, 0, stream_>>>(dm_.nC, z, p, st_);
+                k_cg_pz<T><<<G, TPB, 0, stream_>>>(dm_.nC, z, p, st_);
                 tmark(k, 4);
                 launchCheck("dic_cg_iter", 0);
             });
-            launches_ += (3 + (D.nColours == 1 ? 2 : 2 * D.nColours - 1)) * static_cast<long>(n);
+            launches_ += (3 + dicKernels(D.nColours, tp.shared)) * static_cast<long>(n);
             launched += n;
             chunk = std::min(chunk * 2, 64);
         }
@@ -2558,6 +2600,7 @@ void Ctx::deviceInner(int64_t& u, int64_t& p, int64_t& t) const
 
 void Ctx::iterate(const cfg_simple_controls& ctl, cfg_simple_result& res)
 {
+    const SolveScope scope(device_);
     prepareIterate(ctl);
     std::memset(&res, 0, sizeof res);
     lastTurbInner = 0;
@@ -2588,6 +2631,7 @@ void Ctx::iterate(const cfg_simple_controls& ctl, cfg_simple_result& res)
 /// solveTransientIncompressiblePiso (pisoSolver.cpp:13-237), one time step
 void Ctx::pisoStep(const cfg_piso_controls& ctl, cfg_piso_result& res)
 {
+    const SolveScope scope(device_);
     tally_ = nullptr;
     CFG_CUDA(cudaSetDevice(device_));
     if (!(ctl.dt > 0)) fail(CFG_EINVAL, "PISO: non-positive time step");
@@ -2991,6 +3035,7 @@ void Ctx::poissonAmgApply3(const double* r, double* z, const int32_t done[3], in
 void Ctx::poissonSolve(const double* b, double* x, int method, double tol, int maxIter, int innerMax, double innerTol,
                        double* out)
 {
+    const SolveScope scope(device_);
     tally_ = nullptr;
     // out: inner iterations, outer iterations, converged, true |b-Ax|2/|b|2,
     //      device ms, initial true relative residual

@@ -168,6 +168,7 @@ void Ctx::sparseSolve(int device, int64_t n64, const int64_t* rs, const int64_t*
             if (cols[k] < 0 || cols[k] >= n) fail(CFG_EINVAL, "sparse solve: column out of range");
     }
     CFG_CUDA(cudaSetDevice(device));
+    const SolveScope scope(device);
     if (rs[0] == 0 && residentSolve(device, n, maxRow, rs, cols, vals, b, x, tol, maxIter, method, rep)) return;
     cudaStream_t s;
     CFG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));

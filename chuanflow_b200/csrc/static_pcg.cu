@@ -232,6 +232,7 @@ extern "C" int cfg_pcg_solve_static(int32_t device, int64_t n64, const int32_t* 
             CFG_CUDA(cudaSetDevice(device));
             switched = true;
         }
+        const SolveScope scope(device);
         unsigned char* base = scratchOn(device);
         double* r = reinterpret_cast<double*>(base);
         double* p = reinterpret_cast<double*>(base + kVecBytes);

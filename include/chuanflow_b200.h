@@ -366,6 +366,12 @@ int cfg_sparse_solve(const cfg_ctx* ctx_or_null, int32_t device, int64_t n, cons
  * fields are then unspecified until they are set again, and its next solve
  * starts clean.  Applies to the solves the calling thread starts from now on. */
 int cfg_solver_wait_limit(int64_t cycles);
+/* A context's solve of that size holds every SM for its length, so that
+ * contexts solving at once would take turns.  It therefore runs as kernels per
+ * iteration, beside the others' and with the same bits, while more than `solves`
+ * calls are solving on the device in this process (a negative number: the
+ * default, 1; 0: always).  This thread's solves. */
+int cfg_solver_grid_solves(int32_t solves);
 /* GPU clock cycles that cfg_pcg_solve_static's one-kernel form waits for its
  * blocks to be running at once before the per-iteration kernels take its place
  * (0 or less: the default, about a millisecond); this thread's solves. */
