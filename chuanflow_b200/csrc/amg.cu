@@ -156,7 +156,7 @@ constexpr int kSingleSweeps = 2;  // the class whose V-cycle has one sweep on ev
 /// The class of a nonsymmetric operator by theta = max over rows of
 /// sum_j |a_ij - a_ji| / (2 a_ii), a bound of the imaginary parts of D^-1 A:
 /// Chebyshev sweeps amplify eigenvalues far off the real axis.
-int skewOf(double theta) { return theta <= 0.5 ? 0 : (theta <= 0.9 ? 1 : kSingleSweeps); }
+int skewOf(double theta) { return theta <= 0.5 ? 0 : (theta <= 0.7 ? 1 : kSingleSweeps); }
 
 /// One full wave of a grid-stride row kernel of TPB threads: the SMs times
 /// the blocks of this kernel one SM holds at once (its registers decide),
@@ -1482,7 +1482,11 @@ Coarse<V> coarseOf(const AmgLevel& L)
 /// numpy model, one sweep / four with lo 0.1 / with lo 0.3 / two damped
 /// Jacobi: theta 0.42 45/25/29/37, 0.71 63/57/49/61, 0.83 87/none/70/87, 0.88
 /// 110/none/90/107): class 1 takes lo 0.3, and only on large levels, where
-/// that is a gain over the launches it adds; class 2 keeps single sweeps.
+/// that is a gain over the launches it adds; class 2 keeps single sweeps.  Its
+/// line at theta 0.7, on the GPU (two outer iterations to 1e-10, class 1 /
+/// single sweeps): 320k cells theta 0.65-0.71 85 / 91 ms, 0.74-0.78 105 / 114,
+/// 0.79-0.82 122 / 128, 0.85-0.87 261 / 144 (1575 / 1337 iterations); 292k
+/// cubes 0.63-0.66 69 / 72, 0.70-0.72 77 / 74, 0.78-0.79 83 / 82.
 Smoother smootherOf(const AmgState& a, int skewClass)
 {
     const bool large = a.lv.size() > 1 && a.lv[1].n >= kSellMinRows;

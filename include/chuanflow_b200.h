@@ -437,7 +437,7 @@ int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32
  * (CFG_POISSON_FCG_AMG and the AMG pressure solves: near symmetric), 1 or 2 (one
  * sweep everywhere: the two calls above, and the V-cycle of
  * CFG_POISSON_FCG_AMG_MPNN).  By theta = max over rows of
- * sum_j |a_ij - a_ji| / (2 a_ii): 0 up to 0.5, 1 up to 0.9, else 2. */
+ * sum_j |a_ij - a_ji| / (2 a_ii): 0 up to 0.5, 1 up to 0.7, else 2. */
 int cfg_poisson_amg_cycle(cfg_ctx* ctx, const double* r, double* z, int32_t vectors, int32_t skew_class);
 /* The class of the momentum matrix that the last AMG momentum solve took its
  * hierarchy's values from (0 before the first), for tests. */
