@@ -435,8 +435,9 @@ int cfg_poisson_amg_apply3(cfg_ctx* ctx, const double* r, double* z, const int32
 /* The V-cycle as the solvers apply it to one vector or to three (3 n values),
  * for tests: the sweeps of the coarse levels as for an operator of skew_class 0
  * (CFG_POISSON_FCG_AMG and the AMG pressure solves: near symmetric), 1 or 2 (one
- * sweep everywhere: the two calls above, and the V-cycle of
- * CFG_POISSON_FCG_AMG_MPNN).  By theta = max over rows of
+ * sweep everywhere: the two calls above, the V-cycle of
+ * CFG_POISSON_FCG_AMG_MPNN, and that of the pressure solves when the couplings
+ * which cfg_amg_strength leaves out are below 0.02 of the largest).  By theta = max over rows of
  * sum_j |a_ij - a_ji| / (2 a_ii): 0 up to 0.5, 1 up to 0.7, else 2. */
 int cfg_poisson_amg_cycle(cfg_ctx* ctx, const double* r, double* z, int32_t vectors, int32_t skew_class);
 /* The class of the momentum matrix that the last AMG momentum solve took its
