@@ -134,6 +134,10 @@ constexpr int kDenseMax = 128;
 // operator: one thread per row fills the GPU in one wave there
 constexpr int kSellMinRows = 32768;
 
+// first coarse levels of this many rows or more take four sweeps, not three
+// (smootherOf)
+constexpr int kFourMinRows = 100000;
+
 /// m sweeps whose product is the Chebyshev polynomial of [lo, hi] in D^-1 A
 Sweeps chebyshev(int m, double lo, double hi)
 {
@@ -1505,11 +1509,16 @@ Coarse<V> coarseOf(const AmgLevel& L)
 /// damped Jacobi.  On the 2M-cell channel (B200, one outer iteration to
 /// 1e-12): one sweep 301 ms (1182 momentum component-iterations, 206 pressure
 /// iterations), two 178 ms (595, 131), three 170 ms (533, 101), four on the
-/// first coarse level and two below 159 ms (471, 106); four pay from
-/// kSellMinRows rows on, where a sweep is not a launch's latency
-/// (262k-cell channel 43 -> 32 ms with two, 29.5 with four; 158k-cell PISO
-/// step 10.6 -> 8.6 ms with two, 9.7 with four).  lo: 0.2 for two sweeps and
-/// 0.1 for four; convection narrows the choice (BiCGStab iterations of a
+/// first coarse level and two below 159 ms (471, 106).  Two take the 158k-cell
+/// PISO step from 10.6 to 8.6 ms, four to 9.7.  Three pay from kSellMinRows
+/// rows on, where a sweep is not a launch's latency, and four from kFourMinRows
+/// on (one outer iteration of channels whose cells are long by 1 to 20, gain
+/// over single sweeps in the mean with two / three / four: 282k cells, 36k rows,
+/// 1.19 / 1.18 / 1.10 and in the worst case 1.04 / 0.99 / 0.91, the 262k-cell
+/// channel of cells long by 2.5 44 -> 33 / 30 / 30 ms; 689k cells, 82k rows, 1.29
+/// / 1.31 / 1.25; 1.2M cells, 144k rows, 1.34 / 1.38 / 1.38; 2.1M cells, 250k
+/// rows, 1.48 / 1.54 / 1.57).  lo: 0.2 for two sweeps and
+/// 0.1 for more; convection narrows the choice (BiCGStab iterations of a
 /// numpy model, one sweep / four with lo 0.1 / with lo 0.3 / two damped
 /// Jacobi: theta 0.42 45/25/29/37, 0.71 63/57/49/61, 0.83 87/none/70/87, 0.88
 /// 110/none/90/107): class 1 takes lo 0.3, and only on large levels, where
@@ -1520,10 +1529,12 @@ Coarse<V> coarseOf(const AmgLevel& L)
 /// cubes 0.63-0.66 69 / 72, 0.70-0.72 77 / 74, 0.78-0.79 83 / 82.
 Smoother smootherOf(const AmgState& a, int skewClass)
 {
-    const bool large = a.lv.size() > 1 && a.lv[1].n >= kSellMinRows;
-    if (skewClass == kSingleSweeps || (skewClass == 1 && !large)) return singleSweeps();
+    const int rows = a.lv.size() > 1 ? a.lv[1].n : 0;
+    if (skewClass == kSingleSweeps || (skewClass == 1 && rows < kSellMinRows)) return singleSweeps();
     const double lo2 = skewClass == 1 ? 0.3 : 0.2, lo4 = skewClass == 1 ? 0.3 : 0.1;
-    return Smoother{large ? chebyshev(4, lo4, 1.9) : chebyshev(2, lo2, 1.9), chebyshev(2, lo2, 1.9)};
+    const Sweeps two = chebyshev(2, lo2, 1.9);
+    if (rows < kSellMinRows) return Smoother{two, two};
+    return Smoother{chebyshev(skewClass == 1 || rows >= kFourMinRows ? 4 : 3, lo4, 1.9), two};
 }
 
 /// The level of the fused tail kernel (the last aggregated level, when it is

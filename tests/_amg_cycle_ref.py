@@ -9,6 +9,7 @@ import numpy as np
 import _amg_ref as R
 
 SELL_MIN_ROWS = 32768
+FOUR_MIN_ROWS = 100000
 
 
 def chebyshev(m, lo, hi=1.9):
@@ -17,13 +18,12 @@ def chebyshev(m, lo, hi=1.9):
 
 def weights(rows, skew_class):
     """Per aggregated level (the finest first): its sweeps' weights."""
-    large = len(rows) > 1 and rows[1] >= SELL_MIN_ROWS
-    if skew_class == 2 or (skew_class == 1 and not large):
+    if skew_class == 2 or (skew_class == 1 and rows[1] < SELL_MIN_ROWS):
         first = rest = [0.8]
     else:
         lo2, lo4 = (0.3, 0.3) if skew_class == 1 else (0.2, 0.1)
         rest = chebyshev(2, lo2)
-        first = chebyshev(4, lo4) if large else rest
+        first = rest if rows[1] < SELL_MIN_ROWS else chebyshev(4 if skew_class == 1 or rows[1] >= FOUR_MIN_ROWS else 3, lo4)
     return [[0.8]] + [first] + [rest] * len(rows)
 
 

@@ -2,7 +2,8 @@
 levels -- against its numpy restatement, for one vector and for three, in every
 class of sweeps: ends in the dense solve after level kernels (last aggregated
 level above 1,024 rows), in the one-block and in the clustered last level, and
-first coarse levels on either side of the SELL-32 rule.
+first coarse levels on either side of the SELL-32 and three-sweep rule and of the four-sweep one
+(the largest system).
 
 Tolerance, from the restatement alone: the device and the FP32 restatement add
 in different orders with the same operators, so each is off the same cycle in
@@ -50,7 +51,8 @@ def cycle(case, r, skew_class):
 # system, how it ends, whether the first coarse level is large
 SYSTEMS = [(tets, 3, "dense", False), (tets, 5, "block", False), (tets, 8, "cluster", False), (tets, 10, "dense", False),
            (tets, 13, "block", False), (tets, 20, "cluster", False), (tets, 40, "block", True),
-           (channel, (68, 66, 65), "dense", True), (channel, (80, 78, 76), "dense", True)]
+           (channel, (68, 66, 65), "dense", True), (channel, (80, 78, 76), "dense", True),
+           (channel, (100, 92, 92), "cluster", True)]
 
 
 @pytest.mark.parametrize("make,size,end,large", SYSTEMS, ids=lambda v: getattr(v, "__name__", str(v)))
