@@ -143,6 +143,18 @@ MEASURED_TRAFFIC = {"bi_spmv2": (334.2e6, "all three components; profiles/k_bi_s
                                            "profiles/k_amgv_pre0_channel2M_full.md")}
 
 
+def extra_coarse_passes(N, rows, entries):
+    """What a V-cycle's coarse levels read beyond one sweep on either side, as
+    (matrix bytes, bytes of one vector): a level of m sweeps goes over its FP32
+    CSR 2 m times, not twice, each time with three streams of its rows.  The
+    first coarse level has `rows` N rows and `entries` N entries and four
+    sweeps from 100,000 rows on, three from 32,768 and two below; the levels
+    below it, two sweeps and a seventh of its size in all."""
+    m = 4 if rows * N >= 100_000 else 3 if rows * N >= 32_768 else 2
+    passes = (2 * m - 2) + 2 / 7
+    return passes * 8 * entries * N, passes * 3 * 4 * rows * N
+
+
 def kernel_bytes(N, F, s=8, i=4):
     """Algorithmic bytes of one launch of each solver kernel as (shared,
     per component): every array counted once per read and once per write,
@@ -161,10 +173,13 @@ def kernel_bytes(N, F, s=8, i=4):
     # residual with the member list, the coarse levels, the prolongation:
     # the sweep, the aggregate map and the coarse output read, the
     # correction written) is counted at its finest-level streams plus about
-    # 30% for the coarser levels.
+    # 30% for the coarser levels with one sweep on either side, and the
+    # further sweeps on the channel's first coarse level (plain aggregation:
+    # 0.12 N rows, 1.5 N entries) and below.
     f4 = 4
     sell32 = (N + 2 * F) * 2 * f4 + f4 * N
-    coarse3 = (1.3 * 3 * f4 * N, 1.3 * 3 * f4 * N)
+    sweepMat, sweepVec = extra_coarse_passes(N, 0.12, 1.5)
+    coarse3 = (1.3 * 3 * f4 * N + sweepMat, 1.3 * 3 * f4 * N + sweepVec)
     return {"cg_spmv": (spmv_sym, 0), "cg_update": (7 * s * N, 0), "cg_p": (4 * s * N, 0),
             # invD in; per component r, p, v in, p, z out
             "bi_p": (s * N, 5 * s * N),
@@ -216,9 +231,11 @@ def simple_step_bytes(N, F, Fb, n_orth, it_p, precond, solver_bytes, s=8, i=4):
         # flexible CG: FP64 SpMV + 9 vector streams, and the V-cycle: at the
         # finest level two FP32 SELL passes (value + column per entry, N + 2F
         # entries) and 12 four-byte vector streams; the coarser levels add
-        # about 30% (their rows are 1/7 as many but longer)
+        # about 30% (their rows are 1/7 as many but longer) with one sweep on
+        # either side, and their further sweeps (aggregates by strength of
+        # connection on the channel: 0.17 N rows, 1.7 N entries)
         fine = 2 * (N + 2 * F) * 8 + 12 * 4 * N
-        extra = it_p * (3 * s * N + s * F + 2 * i * F + 9 * s * N + 1.3 * fine)
+        extra = it_p * (3 * s * N + s * F + 2 * i * F + 9 * s * N + 1.3 * fine + sum(extra_coarse_passes(N, 0.17, 1.7)))
     return fixed + solver_bytes + extra
 
 
