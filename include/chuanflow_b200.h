@@ -330,7 +330,9 @@ int cfg_last_timing(const cfg_ctx* ctx, double kernel_ms[8], int64_t* launches);
 
 /* Opt-in CUDA-event timing of every linear-solver kernel launch on the
  * context's stream (no reference counterpart); while it is on, solver
- * iterations are launched one by one rather than as CUDA graphs.  Enabling
+ * iterations are launched one by one rather than as CUDA graphs, and the
+ * Jacobi and DIC solves that otherwise run as one kernel (up to 262,144 rows)
+ * run as the kernels listed here, so it times those, not that one.  Enabling
  * clears the counts; cfg_kernel_stats gives {launches, total ms} for the
  * first `slots` (at most CFG_KERNEL_SLOTS) of, in order: the PCG SpMV +
  * p.Ap, the x/r update + norms + r.z, the search-direction update; the four
