@@ -1939,7 +1939,9 @@ __global__ void __launch_bounds__(TPB) k_fcgd_update_pre0(DMat A, const float* _
 /// update in the first sweep: two launches fewer per iteration for a second
 /// gathered vector in each (158k-cell PISO step 9.5 -> 8.4 ms, 55k-tet Poisson
 /// 3.27 -> 3.16 ms; above it the gathers cost more than the launches: 262k
-/// cells 31.4 -> 31.6 ms, 1.2M 16.4 -> 16.8 ms, 2M 158.7 -> 162.6 ms).
+/// cells 31.4 -> 31.6 ms, 1.2M 16.4 -> 16.8 ms, 2M 158.7 -> 162.6 ms; Poisson
+/// solves of 195k, 216k, 275k and 348k cubes 3.49 -> 3.33, 3.58 -> 3.43, 3.96 ->
+/// 3.92 and 4.42 -> 4.47 ms).
 constexpr int kFormRows = 200000;
 
 }  // namespace

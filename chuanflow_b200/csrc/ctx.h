@@ -462,7 +462,10 @@ private:
     // kPdlRows rows, whose kernels last a few microseconds (55k-tet Poisson
     // 3.02 -> 2.88 ms, 158k-cell PISO step 8.33 -> 7.96 ms); above, the
     // waiting blocks hold the running kernel's slots (262k cells 42.6 -> 43.3
-    // ms, 2M 298 -> 302 ms before the sweeps' change).  CHUANFLOW_PDL=1: on
+    // ms, 2M 298 -> 302 ms before the sweeps' change).  The pressure solve alone
+    // gains beyond the line too: Poisson solves of 195k, 216k, 275k and 348k
+    // cubes 3.33 -> 2.99, 3.43 -> 3.05, 3.96 -> 3.67 and 4.42 -> 4.38 ms; the line
+    // is where the momentum's kernels stop gaining.  CHUANFLOW_PDL=1: on
     // every size, 0: on none.  The results are the same.
     static constexpr int kPdlRows = 200000;
     bool amgPdl() const { return pdl_ < 0 ? dm_.nC <= kPdlRows : pdl_ != 0; }
