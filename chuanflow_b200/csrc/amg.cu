@@ -1517,8 +1517,8 @@ Coarse<V> coarseOf(const AmgLevel& L)
 /// 1.19 / 1.18 / 1.10 and in the worst case 1.04 / 0.99 / 0.91, the 262k-cell
 /// channel of cells long by 2.5 44 -> 33 / 30 / 30 ms; 689k cells, 82k rows, 1.29
 /// / 1.31 / 1.25; 1.2M cells, 144k rows, 1.34 / 1.38 / 1.38; 2.1M cells, 250k
-/// rows, 1.48 / 1.54 / 1.57).  lo: 0.2 for two sweeps and
-/// 0.1 for more; convection narrows the choice (BiCGStab iterations of a
+/// rows, 1.48 / 1.54 / 1.57).  lo: 0.2 for two sweeps and 0.1 for more;
+/// convection narrows the choice (BiCGStab iterations of a
 /// numpy model, one sweep / four with lo 0.1 / with lo 0.3 / two damped
 /// Jacobi: theta 0.42 45/25/29/37, 0.71 63/57/49/61, 0.83 87/none/70/87, 0.88
 /// 110/none/90/107): class 1 takes lo 0.3, and only on large levels, where

@@ -37,6 +37,7 @@ void setTeamWaitLimit(long long cycles);
 /// and those that the blocks of a plain launch wait for all to be there
 /// (cfg_solver_start_limit)
 long long teamStartLimit();
+void setTeamStartLimit(long long cycles);
 /// the solves at once on a device up to which one of them still takes a grid
 /// team (cfg_solver_grid_solves)
 int gridSolvesLimit();
@@ -54,7 +55,6 @@ public:
 private:
     int device_;
 };
-void setTeamStartLimit(long long cycles);
 
 struct Timing
 {
